@@ -1,9 +1,8 @@
 // dense.cu -- FP64 dense block operations of the batched solver:
 //   k_gram        [G | H] = W^H [W | Y]  (partials over row chunks)
 //   k_gram_reduce fixed-order sum of the partials, Hermitian completion
-//   k_small       per problem: column scaling, Cholesky, triangular inverse,
-//                 projected Hermitian matrix, Jacobi eigensolve, sort, C,
-//                 next Chebyshev window and coefficient table
+//   (small.cu: from G and H to the Ritz values, the rotation's coefficients C
+//   and the next Chebyshev window)
 //   k_rotate      V = W C
 //   k_residual64  R = (-Delta) V - V diag(theta) (FP64 stencil), S = -2 c_hop R
 //                 (FP32), residual partial sums
@@ -217,362 +216,6 @@ __global__ void k_gram_reduce(const ProbDesc* __restrict__ pd, const ProbState* 
   }
 }
 
-// ------------------------------------------------------------ small dense --
-// One CTA (1024 threads) per active problem.  Work arrays (column-major k x k)
-// at kk: [0] G -> C, [1] H, [2] Minv, [3] T1 / Q, [4] Ht.
-__device__ __forceinline__ double2& at(double2* M, int k, int i, int j) { return M[i + (size_t)j * k]; }
-
-__global__ void __launch_bounds__(1024) k_small(const ProbDesc* __restrict__ pd, ProbState* __restrict__ ps,
-                                                double2* __restrict__ KK, double* __restrict__ theta,
-                                                double* __restrict__ tcoef, double* __restrict__ scol,
-                                                double* __restrict__ dwork, int first_iter, int fixed_cut,
-                                                int max_sweeps, unsigned long long* __restrict__ tstamp) {
-  const int p = blockIdx.x;
-  if (!ps[p].active) return;
-  // phase boundaries (global timer, ns) for the solver's trace: [p][0..6]
-  auto stamp = [&](int ph) {
-    if (threadIdx.x == 0) {
-      unsigned long long t;
-      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-      tstamp[p * kSmallPhases + ph] = t;
-    }
-  };
-  stamp(0);
-  const ProbDesc d = pd[p];
-  const int k = d.k, tid = threadIdx.x, nt = blockDim.x;
-  // Locked columns [0, c0) (a multiple of the tile width) stay as they are: the
-  // Rayleigh-Ritz runs on the active block a = [c0, k), with W_a projected
-  // against the locked Ritz vectors V_l (= W_l).  n = k - c0; every matrix
-  // below keeps the leading dimension k.
-  const int c0 = ps[p].c0, n = k - c0;
-  const size_t kk2 = (size_t)k * k;
-  double2* G = KK + d.kk;
-  double2* H = G + kk2;
-  double2* Mi = G + 2 * kk2;
-  double2* Q = G + 3 * kk2;
-  double2* Ht = G + 4 * kk2;
-  double2* Ga = G + c0 + (size_t)c0 * k;  // G_aa -> R (scaled Cholesky factor)
-  double2* Ha = H + c0 + (size_t)c0 * k;  // H_aa
-  double* dinv = dwork + d.kv * 4;  // 4 k-length scratch vectors per problem
-  double* lam = dinv + k;
-  int* perm = reinterpret_cast<int*>(lam + k);
-  double* th = theta + d.kv;
-  __shared__ int s_flag;
-  __shared__ double s_red[32];
-  const int nn = n * n;
-
-  // (0) projection against the locked block: with G_la = V_l^H W_a and
-  // H_la = V_l^H A W_a (Gram tiles of the locked rows), V_l^H V_l = I and
-  // V_l^H A V_l = Theta_l,  W_a' = W_a - V_l G_la  has
-  //   G' = G_aa - G_la^H G_la,
-  //   H' = H_aa - G_la^H H_la - H_la^H G_la + G_la^H Theta_l G_la.
-  if (c0 > 0) {
-    for (int e = tid; e < nn; e += nt) {
-      const int i = e % n, j = e / n;
-      const double2* gi = G + (size_t)(c0 + i) * k;
-      const double2* gj = G + (size_t)(c0 + j) * k;
-      const double2* hi = H + (size_t)(c0 + i) * k;
-      const double2* hj = H + (size_t)(c0 + j) * k;
-      double2 sg = make_double2(0.0, 0.0), sh = make_double2(0.0, 0.0);
-      for (int q = 0; q < c0; ++q) {
-        const double2 a = gi[q], b = gj[q];
-        cfmac(sg, a, b);                                 // conj(G_qi) G_qj
-        cfmac(sh, a, hj[q]);                             // conj(G_qi) H_qj
-        cfmac(sh, hi[q], b);                             // conj(H_qi) G_qj
-        const double2 t = cmulc(a, b);
-        sh = make_double2(sh.x - th[q] * t.x, sh.y - th[q] * t.y);  // - theta_q conj(G_qi) G_qj
-      }
-      double2& g = Ga[i + (size_t)j * k];
-      double2& h = Ha[i + (size_t)j * k];
-      g = csub(g, sg);
-      h = csub(h, sh);
-    }
-    __syncthreads();
-  }
-  // (a) column scaling D = sqrt(diag G')
-  for (int i = tid; i < n; i += nt) {
-    const double g = Ga[i + (size_t)i * k].x;
-    dinv[i] = g > 0.0 ? 1.0 / sqrt(g) : 1.0;
-  }
-  if (tid == 0) s_flag = 0;
-  __syncthreads();
-  for (int e = tid; e < nn; e += nt) {
-    const int i = e % n, j = e / n;
-    Ga[i + (size_t)j * k] = cscal(Ga[i + (size_t)j * k], dinv[i] * dinv[j]);
-  }
-  __syncthreads();
-  // (b) Cholesky G' = R^H R, R upper, in place (right-looking)
-  for (int q = 0; q < n; ++q) {
-    if (tid == 0) {
-      double piv = at(Ga, k, q, q).x;
-      if (!(piv > 1e-28)) {
-        piv = 1e-28;
-        s_flag = 1;
-      }
-      at(Ga, k, q, q) = make_double2(sqrt(piv), 0.0);
-    }
-    __syncthreads();
-    const double rinv = 1.0 / at(Ga, k, q, q).x;
-    for (int j = q + 1 + tid; j < n; j += nt) at(Ga, k, q, j) = cscal(at(Ga, k, q, j), rinv);
-    __syncthreads();
-    const int m = n - q - 1;
-    for (int e = tid; e < m * m; e += nt) {
-      const int i = q + 1 + e / m, j = q + 1 + e % m;
-      if (i <= j) {
-        double2 v = at(Ga, k, i, j);
-        const double2 a = at(Ga, k, q, i), b = at(Ga, k, q, j);
-        // v -= conj(a) b
-        v.x -= a.x * b.x + a.y * b.y;
-        v.y -= a.x * b.y - a.y * b.x;
-        at(Ga, k, i, j) = v;
-      }
-    }
-    __syncthreads();
-  }
-  stamp(1);
-  // (c) Minv = D^{-1} R^{-1} (upper triangular), column by column
-  for (int e = tid; e < nn; e += nt) Mi[e % n + (size_t)(e / n) * k] = make_double2(0.0, 0.0);
-  __syncthreads();
-  for (int j = 0; j < n; ++j) {
-    const double rjj = at(Ga, k, j, j).x;
-    for (int i = tid; i <= j; i += nt) {
-      double2 s = make_double2(i == j ? 1.0 : 0.0, 0.0);
-      for (int q = i; q < j; ++q) {
-        // s -= Rinv(i,q) R(q,j)
-        const double2 a = at(Mi, k, i, q), b = at(Ga, k, q, j);
-        s.x -= a.x * b.x - a.y * b.y;
-        s.y -= a.x * b.y + a.y * b.x;
-      }
-      at(Mi, k, i, j) = cscal(s, 1.0 / rjj);
-    }
-    __syncthreads();
-  }
-  for (int e = tid; e < nn; e += nt) {
-    const int i = e % n, j = e / n;
-    Mi[i + (size_t)j * k] = cscal(Mi[i + (size_t)j * k], dinv[i]);
-  }
-  __syncthreads();
-  stamp(2);
-  // (d) T1 = H' Minv ; Ht = Minv^H T1 (Hermitian part)
-  for (int e = tid; e < nn; e += nt) {
-    const int i = e % n, j = e / n;
-    double2 s = make_double2(0.0, 0.0);
-    for (int q = 0; q <= j; ++q) cfma(s, at(Ha, k, i, q), at(Mi, k, q, j));
-    Q[i + (size_t)j * k] = s;
-  }
-  __syncthreads();
-  for (int e = tid; e < nn; e += nt) {
-    const int i = e % n, j = e / n;
-    double2 s = make_double2(0.0, 0.0);
-    for (int q = 0; q <= i; ++q) cfmac(s, at(Mi, k, q, i), at(Q, k, q, j));
-    Ht[i + (size_t)j * k] = s;
-  }
-  __syncthreads();
-  for (int e = tid; e < nn; e += nt) {
-    const int i = e % n, j = e / n;
-    if (i < j) {
-      const double2 a = at(Ht, k, i, j), b = at(Ht, k, j, i);
-      const double2 h = make_double2(0.5 * (a.x + b.x), 0.5 * (a.y - b.y));
-      at(Ht, k, i, j) = h;
-      at(Ht, k, j, i) = cconj(h);
-    } else if (i == j) {
-      at(Ht, k, i, i).y = 0.0;
-    }
-    Q[i + (size_t)j * k] = make_double2(i == j ? 1.0 : 0.0, 0.0);
-  }
-  __syncthreads();
-  stamp(3);
-  // (e) cyclic Jacobi in "position order": in every step position i is paired
-  // with its mirror n-1-i, and after the rotations positions 1..n-1 shift by
-  // one (round-robin tournament: every pair meets once in n-1 steps).  The
-  // shift is folded into the update, which writes the rotated 2x2 blocks of
-  // Ht (and the rotated column pairs of Q) to their new positions in a second
-  // buffer, so each step is one read and one write of both matrices with
-  // unit-stride warp accesses.  Ht ping-pongs with the H storage, Q with the
-  // active block of the G storage (the Cholesky factor, no longer needed);
-  // Q's rows stay in the basis order and its columns follow Ht's diagonal,
-  // which is all the sort below needs.
-  __shared__ double s_c[256], s_s[256];
-  __shared__ double2 s_e[256];
-  const int half = n / 2;
-  double2* hc = Ht;  // current Ht
-  double2* hn = H;   // next Ht
-  double2* qc = Q;
-  double2* qn = Ga;
-  auto shift = [&](int pos) { return pos == 0 ? 0 : (pos == n - 1 ? 1 : pos + 1); };
-  for (int sweep = 0; sweep < max_sweeps; ++sweep) {
-    double off = 0.0, dia = 0.0;
-    for (int e = tid; e < nn; e += nt) {
-      const int i = e % n, j = e / n;
-      const double2 v = hc[i + (size_t)j * k];
-      if (i != j) off += v.x * v.x + v.y * v.y;
-      else dia += v.x * v.x;
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      off += __shfl_xor_sync(0xffffffffu, off, o);
-      dia += __shfl_xor_sync(0xffffffffu, dia, o);
-    }
-    __shared__ double s_off[32], s_dia[32];
-    if ((tid & 31) == 0) {
-      s_off[tid >> 5] = off;
-      s_dia[tid >> 5] = dia;
-    }
-    __syncthreads();
-    if (tid == 0) {
-      double a = 0.0, b = 0.0;
-      for (int w = 0; w < (nt >> 5); ++w) {
-        a += s_off[w];
-        b += s_dia[w];
-      }
-      s_red[0] = a;
-      s_red[1] = b;
-    }
-    __syncthreads();
-    // |off| <= 3e-14 |diag|: with eigenvalue gaps >= 1e-3 lambda_max this
-    // leaves eigenvector errors below 1e-10, far under the residual target
-    if (s_red[0] <= 1e-27 * s_red[1]) break;
-    for (int step = 0; step < n - 1; ++step) {
-      // rotation of pair r = (r, n-1-r): J (p,p)=c (p,q)=s (q,p)=-s e (q,q)=c e, e = e^{-i phi}
-      for (int r = tid; r < half; r += nt) {
-        const int pa = r, qb = n - 1 - r;
-        const double2 g = at(hc, k, pa, qb);
-        const double rr = hypot(g.x, g.y);
-        const double app = at(hc, k, pa, pa).x, aqq = at(hc, k, qb, qb).x;
-        double c = 1.0, s = 0.0;
-        double2 em = make_double2(1.0, 0.0);
-        if (rr > 1e-300 && rr > 1e-18 * sqrt(fabs(app * aqq))) {
-          em = make_double2(g.x / rr, -g.y / rr);
-          const double tau = (aqq - app) / (2.0 * rr);
-          const double tt = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
-          c = 1.0 / sqrt(1.0 + tt * tt);
-          s = tt * c;
-        }
-        s_c[r] = c;
-        s_s[r] = s;
-        s_e[r] = em;
-      }
-      __syncthreads();
-      // Ht <- J^H Ht J on every 2x2 block (rows r', n-1-r'; columns r, n-1-r), shifted
-      for (int e = tid; e < half * half; e += nt) {
-        const int r = e / half, rp = e - r * half;
-        const int p = r, q = n - 1 - r, pp = rp, qq = n - 1 - rp;
-        const double c = s_c[r], s = s_s[r];
-        const double2 em = s_e[r];
-        const double c2 = s_c[rp], s2 = s_s[rp];
-        const double2 ep = cconj(s_e[rp]);
-        const double2 a_pp = at(hc, k, pp, p), a_qp = at(hc, k, qq, p);
-        const double2 a_pq = at(hc, k, pp, q), a_qq = at(hc, k, qq, q);
-        // columns: X = A J
-        const double2 t1 = cmul(a_pq, em), t2 = cmul(a_qq, em);
-        const double2 x_pp = make_double2(c * a_pp.x - s * t1.x, c * a_pp.y - s * t1.y);
-        const double2 x_qp = make_double2(c * a_qp.x - s * t2.x, c * a_qp.y - s * t2.y);
-        const double2 x_pq = make_double2(s * a_pp.x + c * t1.x, s * a_pp.y + c * t1.y);
-        const double2 x_qq = make_double2(s * a_qp.x + c * t2.x, s * a_qp.y + c * t2.y);
-        // rows: B = J'^H X, J'^H (p',p')=c' (p',q')=-s' conj(e') (q',p')=s' (q',q')=c' conj(e')
-        const double2 u1 = cmul(x_qp, ep), u2 = cmul(x_qq, ep);
-        double2 b_pp = make_double2(c2 * x_pp.x - s2 * u1.x, c2 * x_pp.y - s2 * u1.y);
-        double2 b_qp = make_double2(s2 * x_pp.x + c2 * u1.x, s2 * x_pp.y + c2 * u1.y);
-        double2 b_pq = make_double2(c2 * x_pq.x - s2 * u2.x, c2 * x_pq.y - s2 * u2.y);
-        double2 b_qq = make_double2(s2 * x_pq.x + c2 * u2.x, s2 * x_pq.y + c2 * u2.y);
-        if (rp == r) {
-          // diagonal block: the rotated pair is decoupled exactly
-          if (s != 0.0) b_pq = b_qp = make_double2(0.0, 0.0);
-          b_pp.y = 0.0;
-          b_qq.y = 0.0;
-        }
-        const int np_ = shift(p), nq_ = shift(q), npp = shift(pp), nqq = shift(qq);
-        at(hn, k, npp, np_) = b_pp;
-        at(hn, k, nqq, np_) = b_qp;
-        at(hn, k, npp, nq_) = b_pq;
-        at(hn, k, nqq, nq_) = b_qq;
-      }
-      // Q <- Q J, columns shifted
-      for (int e = tid; e < half * n; e += nt) {
-        const int r = e / n, i = e - r * n;
-        const int p = r, q = n - 1 - r;
-        const double c = s_c[r], s = s_s[r];
-        const double2 em = s_e[r];
-        const double2 qp = at(qc, k, i, p), qq = cmul(at(qc, k, i, q), em);
-        at(qn, k, i, shift(p)) = make_double2(c * qp.x - s * qq.x, c * qp.y - s * qq.y);
-        at(qn, k, i, shift(q)) = make_double2(s * qp.x + c * qq.x, s * qp.y + c * qq.y);
-      }
-      __syncthreads();
-      double2* t = hc;
-      hc = hn;
-      hn = t;
-      t = qc;
-      qc = qn;
-      qn = t;
-    }
-  }
-  if (qc != Q) {
-    // bring Q home: its other buffer is written below
-    for (int e = tid; e < nn; e += nt) {
-      const size_t o = e % n + (size_t)(e / n) * k;
-      Q[o] = qc[o];
-    }
-    __syncthreads();
-  }
-  stamp(4);
-  // (f) sort ascending (rank sort, ties by index)
-  for (int i = tid; i < n; i += nt) lam[i] = at(hc, k, i, i).x;
-  __syncthreads();
-  for (int i = tid; i < n; i += nt) {
-    const double li = lam[i];
-    int r = 0;
-    for (int j = 0; j < n; ++j) {
-      const double lj = lam[j];
-      r += (lj < li) || (lj == li && j < i);
-    }
-    perm[r] = i;
-  }
-  __syncthreads();
-  for (int r = tid; r < n; r += nt) th[c0 + r] = lam[perm[r]];
-  // (g) C_a = Minv Q[:, perm]; the rotation's coefficients of the active
-  // columns over the whole block are [-G_la C_a ; C_a] (the V_l part undoes
-  // the projection), stored in columns c0.. of the G storage
-  double2* T = c0 > 0 ? H : Ga;  // C_a (H is free after the sort)
-  for (int e = tid; e < nn; e += nt) {
-    const int i = e % n, j = e / n;
-    const int pj = perm[j];
-    double2 s = make_double2(0.0, 0.0);
-    for (int q = i; q < n; ++q) cfma(s, at(Mi, k, i, q), at(Q, k, q, pj));
-    T[i + (size_t)j * k] = s;
-  }
-  __syncthreads();
-  if (c0 > 0) {
-    // X = -G_la C_a into Ht (free), then both parts into G's columns c0..
-    for (int e = tid; e < c0 * n; e += nt) {
-      const int q = e % c0, j = e / c0;
-      double2 s = make_double2(0.0, 0.0);
-      for (int i = 0; i < n; ++i) cfma(s, G[q + (size_t)(c0 + i) * k], T[i + (size_t)j * k]);
-      Ht[q + (size_t)j * k] = make_double2(-s.x, -s.y);
-    }
-    __syncthreads();
-    for (int e = tid; e < k * n; e += nt) {
-      const int row = e % k, j = e / k;
-      G[row + (size_t)(c0 + j) * k] = row < c0 ? Ht[row + (size_t)j * k] : T[(row - c0) + (size_t)j * k];
-    }
-    __syncthreads();
-  }
-  stamp(5);
-  // (h) next window [lam_cut, lam_max] and Chebyshev coefficients
-  if (tid == 0) {
-    ProbState& S = ps[p];
-    double cut = th[k - 1];
-    if (fixed_cut || (first_iter && S.lam_cut > 0.0)) cut = S.lam_cut;
-    if (cut >= S.lam_max - 1e-3) cut = S.lam_max - 1e-3;
-    if (cut < 1e-6) cut = 1e-6;
-    S.lam_cut = cut;
-    const double al = 2.0 / (S.lam_max - cut);
-    S.c_hop = al;
-    S.c_diag = (S.lam_max + cut - 12.0) / (S.lam_max - cut);
-    S.chol_fail = s_flag;
-    S.theta_min = th[0];
-  }
-  stamp(6);
-}
-
 // ------------------------------------------------- Chebyshev coefficients --
 // Scaled recurrence for a filter of degree m (chosen by the host each
 // iteration).  With E_1 = S/2, E_0 = 0 and
@@ -669,7 +312,7 @@ __global__ void __launch_bounds__(128) k_rotate(const ProbDesc* __restrict__ pd,
   const int row0 = rt * RR, col0 = ct * RC;
   if (col0 < ps[p].c0) return;  // frozen columns keep their Ritz vectors
   const int k = d.k;
-  const double2* C = KK + d.kk;
+  const double2* C = KK + d.kk + 4 * (size_t)k * k;  // the small step's output
   const double2* Wb = Wp + d.blk;
   extern __shared__ double2 rsm[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1035,7 +678,7 @@ int dense_init() {
   LAPH_CUDA_TRY(cudaFuncSetAttribute(k_rotate, cudaFuncAttributeMaxDynamicSharedMemorySize, kRotSmem));
   LAPH_CUDA_TRY(cudaFuncSetAttribute(k_residual64_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, kResidSmem));
   LAPH_TRY(neglap64_init());
-  return LAPH_OK;
+  return small_init();
 }
 int gram(const ProbDesc* pd, const ProbState* ps, const int* start, int np, int nblk, int chunk_rows,
          const double2* W, const double2* Y, double2* gpart, cudaStream_t st) {
@@ -1046,13 +689,6 @@ int gram(const ProbDesc* pd, const ProbState* ps, const int* start, int np, int 
 int gram_reduce(const ProbDesc* pd, const ProbState* ps, const int* start, int np, int nblk, const double2* gpart,
                 double2* KK, cudaStream_t st) {
   k_gram_reduce<<<nblk, 256, 0, st>>>(pd, ps, start, np, gpart, KK);
-  LAPH_CUDA_TRY(cudaGetLastError());
-  return LAPH_OK;
-}
-int small_dense(const ProbDesc* pd, ProbState* ps, int np, double2* KK, double* theta, double* tcoef, double* scol,
-                double* dwork, int first_iter, int fixed_cut, int max_sweeps, unsigned long long* tstamp,
-                cudaStream_t st) {
-  k_small<<<np, 1024, 0, st>>>(pd, ps, KK, theta, tcoef, scol, dwork, first_iter, fixed_cut, max_sweeps, tstamp);
   LAPH_CUDA_TRY(cudaGetLastError());
   return LAPH_OK;
 }

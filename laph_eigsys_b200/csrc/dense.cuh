@@ -11,12 +11,16 @@ int gram(const ProbDesc* pd, const ProbState* ps, const int* start, int np, int 
          const double2* W, const double2* Y, double2* gpart, cudaStream_t st);
 int gram_reduce(const ProbDesc* pd, const ProbState* ps, const int* start, int np, int nblk, const double2* gpart,
                 double2* KK, cudaStream_t st);
-// Per problem: scaling, Cholesky, inverse, projected matrix, Jacobi, sort, C, next window.
-// tstamp[p][0..kSmallPhases-1] receives the global timer (ns) at the phase boundaries.
+// Per problem, from G and H: projection against the frozen columns, Cholesky, inverse, projected matrix, Jacobi
+// (at most max_sweeps sweeps), sort, the rotation's coefficients C (fifth k x k matrix of KK), next window
+// (small.cu); kmax: the batch's widest block.  tstamp[p][0..kSmallPhases-1] receives the global timer (ns) at the
+// phase boundaries.
 constexpr int kSmallPhases = 7;
-int small_dense(const ProbDesc* pd, ProbState* ps, int np, double2* KK, double* theta, double* tcoef, double* scol,
-                double* dwork, int first_iter, int fixed_cut, int max_sweeps, unsigned long long* tstamp,
-                cudaStream_t st);
+int small_init();
+int small_dense(const ProbDesc* pd, ProbState* ps, int np, int kmax, double2* KK, double* theta, double* dwork,
+                int first_iter, int fixed_cut, int max_sweeps, unsigned long long* tstamp, cudaStream_t st);
+// kernels one small_dense call launches
+int small_launches(int kmax, int max_sweeps);
 // Chebyshev coefficient table and S scaling for a filter of degree m (or *dm
 // when dm is not null: the degree the device-side loop chose).
 int coef(const ProbDesc* pd, const ProbState* ps, int np, const double* theta, double* tcoef, double* scol, int m,

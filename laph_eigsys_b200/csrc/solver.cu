@@ -53,6 +53,7 @@ struct laph_solver {
   cudaStream_t st = nullptr;
   laph_solve_opts o{};
   int np = 0, mdeg = 16, kb = 32, tile = 128;
+  int kmax = 0;                // widest block of the batch
   int fvariant = 1, lmax = 0;  // filter variant in use (opts.filter_kernel, or 1 where 3 does not apply)
   int* d_ferr = nullptr;       // set by the staged filter when a pipeline wait gives up
   std::vector<ProbDesc> hd;
@@ -310,6 +311,7 @@ int laph_solver_create(laph_solver** out, const laph_problem* probs, int n, cons
     o_rp += (long long)d.nrt * d.k;
     o_tc += (long long)(s->mdeg + 1) * 3 * d.k;
     s->hd.push_back(d);
+    s->kmax = std::max(s->kmax, d.k);
     max_v3 = std::max(max_v3, (size_t)d.V3);
     const int nst = (d.V3 + 127) / 128;
     per_site.push_back(nst);
@@ -450,13 +452,17 @@ static int residual(laph_solver* s) {
   return residual64_cols(s->d_pd, s->d_ps, s->st_nl, s->np, s->nb_nl, s->U64, s->V, s->theta, s->S, s->rpart, s->st);
 }
 
+static int jacobi_sweeps(const laph_solver* s) { return s->o.jacobi_sweeps > 0 ? s->o.jacobi_sweeps : 2; }
+// kernels of one iteration_rr: A W, Gram, its reduction, the small step, rotation, residual, zero, check
+static long long rr_launches(const laph_solver* s) { return 7 + small_launches(s->kmax, jacobi_sweeps(s)); }
+
 static int iteration_rr(laph_solver* s, int first_iter) {
   const bool fixed = s->o.window == LAPH_WINDOW_FIXED && s->o.lam_cut > 0.0;
   LAPH_TRY(neglap64_batch(s->d_pd, s->d_ps, s->st_nl, s->np, s->nb_nl, s->U64, s->W, s->Y, s->st));
   LAPH_TRY(gram(s->d_pd, s->d_ps, s->st_gram, s->np, s->nb_gram, 8192, s->W, s->Y, s->gpart, s->st));
   LAPH_TRY(gram_reduce(s->d_pd, s->d_ps, s->st_gred, s->np, s->nb_gred, s->gpart, s->KK, s->st));
-  LAPH_TRY(small_dense(s->d_pd, s->d_ps, s->np, s->KK, s->theta, s->tcoef, s->scol, s->dwork, first_iter, fixed ? 1 : 0,
-                       s->o.jacobi_sweeps > 0 ? s->o.jacobi_sweeps : 2, s->tstamp, s->st));
+  LAPH_TRY(small_dense(s->d_pd, s->d_ps, s->np, s->kmax, s->KK, s->theta, s->dwork, first_iter, fixed ? 1 : 0,
+                       jacobi_sweeps(s), s->tstamp, s->st));
   LAPH_TRY(rotate(s->d_pd, s->d_ps, s->st_rot, s->np, s->nb_rot, s->W, s->KK, s->V, s->st));
   LAPH_TRY(residual(s));
   LAPH_TRY(zero_int(s->d_nactive, s->st));
@@ -590,7 +596,7 @@ static int solve_setup(laph_solver* s, bool device_loop, long long* nlaunch_out)
     LAPH_TRY(random_block(s->d_pd, s->st_rand, s->np, s->nb_rand, s->W, o.seed, s->st));
     if (!device_loop) LAPH_CUDA_TRY(cudaEventRecord(s->ev1, s->st));
     LAPH_TRY(iteration_rr(s, 1));
-    nlaunch += 2 + 8;  // pack, random block, first Rayleigh-Ritz
+    nlaunch += 2 + rr_launches(s);  // pack, random block, first Rayleigh-Ritz
   }
   *nlaunch_out = nlaunch;
   return LAPH_OK;
@@ -800,9 +806,8 @@ static int run_device_loop(laph_solver* s, laph_result* res) {
   for (int m : s->degs) fl += m - 1;
   s->cnt[0] = (long long)ls.sv_steps;
   s->cnt[1] = fl;
-  // per pass: loop_pass_begin, coef, direct_start, the m - 1 steps, loop_pass_end, 8 Rayleigh-Ritz kernels,
-  // loop_cond
-  s->cnt[2] = s->solve_setup_launches + 13LL * ls.npass + fl;
+  // per pass: loop_pass_begin, coef, direct_start, the m - 1 steps, loop_pass_end, Rayleigh-Ritz, loop_cond
+  s->cnt[2] = s->solve_setup_launches + (5 + rr_launches(s)) * ls.npass + fl;
   s->fbytes[0] = ls.fbytes[0];
   s->fbytes[1] = ls.fbytes[1];
   s->ran = 1;
@@ -979,7 +984,7 @@ int laph_solver_run(laph_solver* s, laph_result* res) {
     LAPH_TRY(filter_graph(s, m, nos));
     LAPH_CUDA_TRY(cudaEventRecord(s->evf[1], s->st));
     LAPH_TRY(rr_graph(s));
-    nlaunch += 2 + (m - 1) + 8;
+    nlaunch += 2 + (m - 1) + rr_launches(s);
     float f = 0.f;
     LAPH_CUDA_TRY(cudaEventSynchronize(s->evf[1]));
     LAPH_CUDA_TRY(cudaEventElapsedTime(&f, s->evf[0], s->evf[1]));
