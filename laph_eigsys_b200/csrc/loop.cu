@@ -111,10 +111,12 @@ __global__ void k_loop_pass_begin(const ProbDesc* __restrict__ pd, ProbState* __
   }
   // the filter steps of this pass: n = 1..m-2 middle (0), n = m-1 the last (1), the same without S (2, 3) for
   // n >= 3 of an all-direct pass, none beyond (4: past the last branch of every SWITCH)
-  for (int n = 1 + tid; n < lp.mdeg; n += blockDim.x) {
-    const unsigned base = n < m - 1 ? 0u : (n == m - 1 ? 1u : 4u);
-    cudaGraphSetConditional(steps[n], base < 2u && nos && n >= 3 ? base + 2u : base);
-  }
+  // (steps null: the pass is one kernel that reads the degree itself)
+  if (steps)
+    for (int n = 1 + tid; n < lp.mdeg; n += blockDim.x) {
+      const unsigned base = n < m - 1 ? 0u : (n == m - 1 ? 1u : 4u);
+      cudaGraphSetConditional(steps[n], base < 2u && nos && n >= 3 ? base + 2u : base);
+    }
   __syncthreads();
   if (tid == 0) {
     ls->it = it;

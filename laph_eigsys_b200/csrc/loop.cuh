@@ -44,7 +44,7 @@ int loop_init(LoopState* ls, const int* wdeg, int np, cudaStream_t st);
 // each problem's direct flag, the counters, and the SWITCH handles of the
 // filter steps n = 1..mdeg-1: 0 = a middle step (n < m - 1), 1 = the last step
 // (n = m - 1), 2 / 3 = the same without S (n >= 3 of a pass every active
-// problem runs directly), 4 = no step.
+// problem runs directly), 4 = no step.  steps may be null (no step nodes).
 int loop_pass_begin(const ProbDesc* pd, ProbState* ps, int np, LoopState* ls, int* degs, double* lam_max0,
                     int* fallback, const cudaGraphConditionalHandle* steps, const LoopParams& lp, cudaStream_t st);
 // End of the filter part of a pass: accumulate its time.

@@ -33,6 +33,7 @@
 #include "common.cuh"
 #include "dense.cuh"
 #include "filter.cuh"
+#include "filter_pass.cuh"
 #include "links.cuh"
 #include "loop.cuh"
 #include "mlp.cuh"
@@ -55,7 +56,9 @@ struct laph_solver {
   int np = 0, mdeg = 16, kb = 32, tile = 128;
   int kmax = 0;                // widest block of the batch
   int fvariant = 1, lmax = 0;  // filter variant in use (opts.filter_kernel, or 1 where 3 does not apply)
-  int* d_ferr = nullptr;       // set by the staged filter when a pipeline wait gives up
+  int* d_ferr = nullptr;       // set by a filter kernel whose bounded wait gave up
+  std::vector<PassClass> pass; // layout of the one-kernel filter pass (empty: one kernel per step)
+  int* d_plan = nullptr;       // its plan and team counters
   std::vector<ProbDesc> hd;
   ProbDesc* d_pd = nullptr;
   ProbState* d_ps = nullptr;
@@ -194,7 +197,7 @@ int laph_solver_destroy(laph_solver* s) {
                   s->st_col, s->U64raw, s->U64, s->Utmp, s->dec, s->stage, s->Uf32, s->Ubf, s->scale, s->V, s->W, s->Y, s->S, s->E[0],
                   s->E[1], s->E[2], s->KK, s->gpart, s->rpart, s->theta, s->tcoef, s->scol, s->dwork, s->resid,
                   s->phases, s->norms, s->d_nactive, s->model, s->feats, s->mwork, s->bound, s->plaq, s->wdeg,
-                  s->tstamp, s->ls, s->d_degs, s->d_lam_max0, s->d_fallback, s->d_steps, s->d_ps0, s->d_ferr};
+                  s->tstamp, s->ls, s->d_degs, s->d_lam_max0, s->d_fallback, s->d_steps, s->d_ps0, s->d_ferr, s->d_plan};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (s->h_nactive) cudaFreeHost(s->h_nactive);
@@ -257,7 +260,11 @@ int laph_solver_create(laph_solver** out, const laph_problem* probs, int n, cons
   s->o = *opts;
   s->np = n;
   s->mdeg = opts->deg;
-  s->kb = opts->block > 0 ? opts->block : 32;
+  // Columns per CTA: 32 unless told otherwise, 16 where 32 would leave too few CTAs per step (below 8e6 site-columns;
+  // 24^3 x 2 and 32^3 x 1, 160 columns: 4.1e10 against 3.9e10 site-columns a second, 32^3 x 2: 4.6e10 either way)
+  long long work = 0;
+  for (int i = 0; i < n; ++i) work += (long long)probs[i].L * probs[i].L * probs[i].L * round_up(probs[i].nev + opts->guard, kGramTile);
+  s->kb = opts->block > 0 ? opts->block : work < 8000000 ? 16 : 32;
   // sites per CTA of the filter; the per-thread-coefficient variant and blocks wider than 64 keep 128
   s->tile = opts->filter_tile > 0 && opts->filter_kernel >= 1 && s->kb <= 64 ? opts->filter_tile : 128;
   // the staged variant (3) needs 128-site tiles of whole z-rows inside one plane for every problem
@@ -347,9 +354,12 @@ int laph_solver_create(laph_solver** out, const laph_problem* probs, int n, cons
       (rc = dalloc(&s->tstamp, (size_t)n * kSmallPhases)) || (rc = dalloc(&s->ls, 1)) ||
       (rc = dalloc(&s->d_degs, (size_t)opts->max_it + 2)) || (rc = dalloc(&s->d_lam_max0, n)) ||
       (rc = dalloc(&s->d_fallback, n)) || (rc = dalloc(&s->d_steps, (size_t)s->mdeg + 1)) ||
-      (rc = dalloc(&s->d_ps0, n)) || (rc = dalloc(&s->d_ferr, 1)))
+      (rc = dalloc(&s->d_ps0, n)) || (rc = dalloc(&s->d_ferr, 1)) || (rc = dalloc(&s->d_plan, pass_plan_ints(n))))
     return fail(rc);
   if (cudaMemset(s->d_ferr, 0, sizeof(int)) != cudaSuccess) return fail(LAPH_ECUDA);
+  // the default filter runs a whole pass as one kernel per extent where the batch is small
+  if (s->fvariant == 1 && s->kb <= 64)
+    if (int e = pass_layout(s->hd, opts->link_prec == LAPH_LINKS_BF16, &s->pass)) return fail(e);
   if (opts->link_prec == LAPH_LINKS_BF16) {
     if ((rc = dalloc(reinterpret_cast<float2**>(&s->Ubf), (size_t)o_uf))) return fail(rc);  // 4 B per element
   } else {
@@ -482,9 +492,21 @@ static int filter_step(laph_solver* s, int n, bool fin, bool nos, cudaStream_t s
                    s->W, s->tcoef, n, fin, s->fvariant, s->tile, s->lmax, s->d_ferr, nos && n >= 3, st);
 }
 
+// All steps of a pass in one kernel per extent (filter_pass.cu), of degree m or *dm.
+static int filter_one(laph_solver* s, int m, const int* dm) {
+  const int bf = s->o.link_prec == LAPH_LINKS_BF16;
+  const void* links = bf ? s->Ubf : static_cast<const void*>(s->Uf32);
+  return filter_pass(s->pass, s->d_pd, s->d_ps, s->np, bf, links, s->scale, s->S, s->E[0], s->E[1], s->V, s->W, s->tcoef,
+                     m, dm, s->d_plan, s->d_ferr, s->st);
+}
+
+// filter kernels a pass of degree m launches
+static long long filter_launches(const laph_solver* s, int m) { return s->pass.empty() ? m - 1 : pass_launches(s->pass); }
+
 static int filter(laph_solver* s, int m, bool nos) {
   LAPH_TRY(coef(s->d_pd, s->d_ps, s->np, s->theta, s->tcoef, s->scol, m, nullptr, s->st));
   LAPH_TRY(direct_start(s->d_pd, s->d_ps, s->st_filt, s->np, s->nb_filt, s->kb, s->tile, s->V, s->S, s->st));
+  if (!s->pass.empty()) return filter_one(s, m, nullptr);
   for (int n = 1; n < m; ++n) LAPH_TRY(filter_step(s, n, n == m - 1, nos, s->st));
   return LAPH_OK;
 }
@@ -606,11 +628,12 @@ static int solve_setup(laph_solver* s, bool device_loop, long long* nlaunch_out)
 static int fill_results(laph_solver* s, laph_result* res) {
   const laph_solve_opts& o = s->o;
   int status = LAPH_OK;
-  if (s->fvariant == 3) {
+  if (s->fvariant == 3 || !s->pass.empty()) {
     int ferr = 0;
     if (cudaMemcpy(&ferr, s->d_ferr, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return LAPH_ECUDA;
     if (ferr != 0) {
-      set_error("laph_solver_run: the staged filter's copy pipeline failed (code %d); results are invalid", ferr);
+      cudaMemset(s->d_ferr, 0, sizeof(int));
+      set_error("laph_solver_run: a bounded wait of the filter gave up (code %d); results are invalid", ferr);
       return LAPH_ECUDA;
     }
   }
@@ -644,7 +667,8 @@ static int fill_results(laph_solver* s, laph_result* res) {
 //   WHILE (any problem active and it < max_it):
 //       loop_pass_begin (degree, the learned window's check, counters, step switches)
 //       coef (degree read on the device)
-//       SWITCH per filter step n = 1..mdeg-1: {plain step n | last step n | nothing}
+//       the filter pass in one kernel per extent (degree read on the device), or, where it does not apply,
+//       a SWITCH per filter step n = 1..mdeg-1: {plain step n | last step n | nothing}
 //       loop_pass_end, Rayleigh-Ritz + residuals + convergence mask, loop_cond
 //   loop_end -> phase fix
 // so no host round trip separates the passes (the host loop reads the mask
@@ -729,9 +753,10 @@ static int build_solve_graph(laph_solver* s) {
   cudaGraph_t body;
   if ((rc = add_conditional(g, deps, h_loop, cudaGraphCondTypeWhile, 1, &body)) != LAPH_OK) return done(rc);
   std::vector<cudaGraphNode_t> top = deps;  // the WHILE node
-  // the pass: one SWITCH handle per filter step position
+  // the pass as step kernels: one SWITCH handle per filter step position
+  const int nswitch = s->pass.empty() ? s->mdeg : 0;
   std::vector<cudaGraphConditionalHandle> hs(s->mdeg + 1, 0);
-  for (int n = 1; n < s->mdeg; ++n)
+  for (int n = 1; n < nswitch; ++n)
     if (cudaGraphConditionalHandleCreate(&hs[n], body, 4, 0) != cudaSuccess) {
       set_error("conditional graph nodes not available");
       return done(LAPH_ECUDA);
@@ -740,14 +765,15 @@ static int build_solve_graph(laph_solver* s) {
     return done(LAPH_ECUDA);
   std::vector<cudaGraphNode_t> bd;
   rc = capture_into(s, body, bd, [&]() -> int {
-    LAPH_TRY(loop_pass_begin(s->d_pd, s->d_ps, s->np, s->ls, s->d_degs, s->d_lam_max0, s->d_fallback, s->d_steps,
-                             lp, s->st));
+    LAPH_TRY(loop_pass_begin(s->d_pd, s->d_ps, s->np, s->ls, s->d_degs, s->d_lam_max0, s->d_fallback,
+                             nswitch ? s->d_steps : nullptr, lp, s->st));
     LAPH_TRY(coef(s->d_pd, s->d_ps, s->np, s->theta, s->tcoef, s->scol, 0, &s->ls->m, s->st));
-    return direct_start(s->d_pd, s->d_ps, s->st_filt, s->np, s->nb_filt, s->kb, s->tile, s->V, s->S, s->st);
+    LAPH_TRY(direct_start(s->d_pd, s->d_ps, s->st_filt, s->np, s->nb_filt, s->kb, s->tile, s->V, s->S, s->st));
+    return nswitch ? LAPH_OK : filter_one(s, 0, &s->ls->m);
   });
   if (rc != LAPH_OK) return done(rc);
   // SWITCH per step position: middle / last step, and for n >= 3 the same two without S
-  for (int n = 1; n < s->mdeg; ++n) {
+  for (int n = 1; n < nswitch; ++n) {
     const unsigned nb = n >= 3 ? 4u : 2u;
     cudaGraph_t b[4];
     if ((rc = add_conditional(body, bd, hs[n], cudaGraphCondTypeSwitch, nb, b)) != LAPH_OK) return done(rc);
@@ -803,10 +829,10 @@ static int run_device_loop(laph_solver* s, laph_result* res) {
   s->ms[3] = b;
   s->ms[2] = b - s->ms[0] - s->ms[1];
   long long fl = 0;
-  for (int m : s->degs) fl += m - 1;
+  for (int m : s->degs) fl += filter_launches(s, m);
   s->cnt[0] = (long long)ls.sv_steps;
   s->cnt[1] = fl;
-  // per pass: loop_pass_begin, coef, direct_start, the m - 1 steps, loop_pass_end, Rayleigh-Ritz, loop_cond
+  // per pass: loop_pass_begin, coef, direct_start, the filter, loop_pass_end, Rayleigh-Ritz, loop_cond
   s->cnt[2] = s->solve_setup_launches + (5 + rr_launches(s)) * ls.npass + fl;
   s->fbytes[0] = ls.fbytes[0];
   s->fbytes[1] = ls.fbytes[1];
@@ -977,14 +1003,14 @@ int laph_solver_run(laph_solver* s, laph_result* res) {
       s->fbytes[0] += (double)d.V3 * (nact * per + nl * 96.0 + (double)nblk * (m - 1) * lbytes);
       s->fbytes[1] += (double)d.V3 * (m - 1) * (nact * 72.0 + (double)nblk * lbytes);
     }
-    s->cnt[1] += m - 1;
+    s->cnt[1] += filter_launches(s, m);
     s->degs.push_back(m);
     if (trace) std::fprintf(stderr, "laph_trace it %d filter degree %d direct %d/%d\n", it, m, ndir_p, nact_p);
     LAPH_CUDA_TRY(cudaEventRecord(s->evf[0], s->st));
     LAPH_TRY(filter_graph(s, m, nos));
     LAPH_CUDA_TRY(cudaEventRecord(s->evf[1], s->st));
     LAPH_TRY(rr_graph(s));
-    nlaunch += 2 + (m - 1) + rr_launches(s);
+    nlaunch += 2 + filter_launches(s, m) + rr_launches(s);
     float f = 0.f;
     LAPH_CUDA_TRY(cudaEventSynchronize(s->evf[1]));
     LAPH_CUDA_TRY(cudaEventElapsedTime(&f, s->evf[0], s->evf[1]));
@@ -1307,6 +1333,7 @@ int laph_solver_footprint(const laph_problem* probs, int n, const laph_solve_opt
   add(o_tc * 8);
   add(4 * o_kv * 8);                          // dwork
   add(4);                                     // active count
+  add((long long)pass_plan_ints(n) * 4);      // plan of the one-kernel filter pass
   add((long long)(kMlpParams + kMlpNorm) * 4);
   add((long long)n * kMlpIn * 4);
   add((long long)n * (kMlpIn + kMlpOut) * 4);
