@@ -179,6 +179,106 @@ __global__ void __launch_bounds__(64) k_gram(const ProbDesc* __restrict__ pd, co
 }
 
 
+// The same partial products for batches with few (tile pair, chunk) units: there
+// the two warps of a unit run 16 MMA tiles' chains on two of an SM's four FP64
+// tensor pipes, 2 us per 16-row stage however idle the chip is (647 us for the
+// 250 stages of 11^3).  Here a CTA of four warps takes a 32 x 16 half of G or of H
+// of a unit, one m16n8k16 tile per warp: four times the CTAs, a quarter of the
+// chain on each pipe, and a six-stage ring so that the loads run ahead of the
+// shorter stages.  Every output element sees the same MMAs in the same order.
+constexpr int GSS = 6, kGramSplitStage = (GT + GT / 2) * GP;  // stages; double2 per stage
+// Up to this many units (of 32^3: 6 timeslices of block width 160, 3 of 224).  Four Rayleigh-Ritz steps, ms, merged ->
+// split: 11^3 k 64 (3 units) 3.41 -> 1.86, 16^3 k 96 (12) 6.17 -> 2.98, 24^3 k 160 (90) 9.74 -> 7.29, 24^3 x 6 (540)
+// 19.6 -> 18.7; a mixed batch of 990 units 85 -> 80 ms per solve; 2160 units (32^3 x 12) and 2952 (48^3 x 2, k 256):
+// no difference or 1% the other way, for twice the reads from L2.
+constexpr int kGramSplitUnits = 1200;
+constexpr int kGramSplitSmem = GSS * kGramSplitStage * (int)sizeof(double2);
+
+__global__ void __launch_bounds__(128) k_gram_split(const ProbDesc* __restrict__ pd, const ProbState* __restrict__ ps,
+                                                    const int* __restrict__ start, int np, int chunk_rows,
+                                                    const double2* __restrict__ W, const double2* __restrict__ Y,
+                                                    double2* __restrict__ gpart) {
+  const int unit = blockIdx.x >> 2, which = (blockIdx.x >> 1) & 1, half = blockIdx.x & 1;
+  const int p = find_prob(start, np, unit);
+  if (!ps[p].active) return;
+  const ProbDesc d = pd[p];
+  const int T = d.k / GT;
+  const int npair = T * (T + 1) / 2;
+  const int t = unit - start[p];
+  const int chunk = t / npair;
+  const int pair = t - chunk * npair;
+  int pr = pair, ti = 0;
+  while (pr >= T - ti) {
+    pr -= T - ti;
+    ++ti;
+  }
+  const int tj = LAPH_IX(ti + pr, T);
+  if ((tj + 1) * GT <= ps[p].c0) return;  // both tiles frozen: not needed
+  const double2* A = W + d.blk + (size_t)(ti * GT) * d.dim;
+  const double2* B = (which ? Y : W) + d.blk + (size_t)(tj * GT + half * (GT / 2)) * d.dim;
+  const int r0 = chunk * chunk_rows, r1 = min(d.dim, r0 + chunk_rows);
+  extern __shared__ double2 gsm[];
+  auto load = [&](int st) {
+    double2* s = gsm + (st % GSS) * kGramSplitStage;
+    const int row = r0 + st * GK + (threadIdx.x & 15);
+    const bool ok = row < r1;
+#pragma unroll
+    for (int e = 0; e < 6; ++e) {
+      const int c = (threadIdx.x >> 4) + 8 * e;  // 32 columns of W_ti, then 16 of W_tj or Y_tj
+      const double2* src = e < 4 ? A + (size_t)c * d.dim : B + (size_t)(c - GT) * d.dim;
+      cp_async16(s + LAPH_IX(gsw(c, threadIdx.x & 15), kGramSplitStage), src + (ok ? row : 0), ok);
+    }
+    cp_async_commit();
+  };
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane >> 2, t4 = lane & 3;
+  const int i = warp & 1, j = warp >> 1;  // 16-row and 8-column tile of this warp
+  const bool skip = ti == tj && i == 1 && half == 0;  // entirely below the diagonal: not kept
+  double accr[4] = {0.0, 0.0, 0.0, 0.0}, acci[4] = {0.0, 0.0, 0.0, 0.0};
+  const int nstep = (r1 - r0 + GK - 1) / GK;
+#pragma unroll
+  for (int st = 0; st < GSS - 1; ++st) {
+    if (st < nstep) load(st);
+    else cp_async_commit();
+  }
+  for (int it = 0; it < nstep; ++it) {
+    cp_async_wait<GSS - 2>();
+    __syncthreads();
+    if (it + GSS - 1 < nstep) load(it + GSS - 1);
+    else cp_async_commit();
+    if (skip) continue;
+    const double2* sA = gsm + (it % GSS) * kGramSplitStage;
+    double ar[8], ai[8], br[4], bi[4], bn[4];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const double2 a = sA[gsw(16 * i + g + 8 * (r & 1), t4 + 4 * (r >> 1))];
+      ar[r] = a.x;
+      ai[r] = a.y;
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const double2 v = sA[gsw(GT + 8 * j + g, t4 + 4 * r)];
+      br[r] = v.x;
+      bi[r] = v.y;
+      bn[r] = -v.x;
+    }
+    dmma16816(accr, ar, br);
+    dmma16816(acci, ar, bi);
+    dmma16816(accr, ai, bi);
+    dmma16816(acci, ai, bn);
+  }
+  cp_async_wait<0>();
+  if (skip) return;
+  double2* o = gpart + d.gp + ((size_t)(chunk * 2 + which) * npair + pair) * (GT * GT);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    if (ti == tj && 2 * i + h > 2 * half + j) continue;
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+      o[(16 * i + 8 * h + g) * GT + 16 * half + 8 * j + 2 * t4 + e] = make_double2(accr[2 * h + e], acci[2 * h + e]);
+  }
+}
+
 // Sum partials (fixed order) and complete the Hermitian matrices G, H
 // (column-major k x k at kk and kk + k*k).
 __global__ void k_gram_reduce(const ProbDesc* __restrict__ pd, const ProbState* __restrict__ ps,
@@ -675,6 +775,7 @@ int to_reference(const double2* in, double2* out, int V3, int nev, cudaStream_t 
 }
 int dense_init() {
   LAPH_CUDA_TRY(cudaFuncSetAttribute(k_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, kGramSmem));
+  LAPH_CUDA_TRY(cudaFuncSetAttribute(k_gram_split, cudaFuncAttributeMaxDynamicSharedMemorySize, kGramSplitSmem));
   LAPH_CUDA_TRY(cudaFuncSetAttribute(k_rotate, cudaFuncAttributeMaxDynamicSharedMemorySize, kRotSmem));
   LAPH_CUDA_TRY(cudaFuncSetAttribute(k_residual64_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, kResidSmem));
   LAPH_TRY(neglap64_init());
@@ -682,7 +783,10 @@ int dense_init() {
 }
 int gram(const ProbDesc* pd, const ProbState* ps, const int* start, int np, int nblk, int chunk_rows,
          const double2* W, const double2* Y, double2* gpart, cudaStream_t st) {
-  k_gram<<<nblk, 64, kGramSmem, st>>>(pd, ps, start, np, chunk_rows, W, Y, gpart);
+  if (nblk <= kGramSplitUnits)
+    k_gram_split<<<4 * nblk, 128, kGramSplitSmem, st>>>(pd, ps, start, np, chunk_rows, W, Y, gpart);
+  else
+    k_gram<<<nblk, 64, kGramSmem, st>>>(pd, ps, start, np, chunk_rows, W, Y, gpart);
   LAPH_CUDA_TRY(cudaGetLastError());
   return LAPH_OK;
 }
