@@ -6,6 +6,8 @@
 // separate output (Jacobi-style, all links updated at once), exactly as the
 // reference's eigen_timeslice_ts temporaries do.  A batch of nts timeslices
 // of equal volume is processed by one launch (grid.y = timeslice).
+#include <utility>
+
 #include "smear.cuh"
 #include "su3.cuh"
 
@@ -152,6 +154,7 @@ int smear_batch(double2* U, double2* Utmp, double2* dec, int L, int nts, int kin
   const size_t dec_stride = (size_t)54 * g.V3;
   if (kind == LAPH_SMEAR_NONE || iters <= 0) return LAPH_OK;
   const dim3 blk(128);
+  double2* const home = U;
   for (int it = 0; it < iters; ++it) {
     if (kind == LAPH_SMEAR_STOUT) {
       k_stout<<<dim3(ceil_div(3LL * g.V3, 128), nts), blk, 0, st>>>(U, Utmp, g, p1, compat, ts_stride);
@@ -169,8 +172,10 @@ int smear_batch(double2* U, double2* Utmp, double2* dec, int L, int nts, int kin
       return LAPH_EINVAL;
     }
     LAPH_CUDA_TRY(cudaGetLastError());
-    LAPH_CUDA_TRY(cudaMemcpyAsync(U, Utmp, sizeof(double2) * ts_stride * nts, cudaMemcpyDeviceToDevice, st));
+    std::swap(U, Utmp);
   }
+  if (U != home)  // an odd number of iterations ends in the other buffer
+    LAPH_CUDA_TRY(cudaMemcpyAsync(home, U, sizeof(double2) * ts_stride * nts, cudaMemcpyDeviceToDevice, st));
   return LAPH_OK;
 }
 

@@ -354,12 +354,14 @@ int laph_solver_create(laph_solver** out, const laph_problem* probs, int n, cons
       (rc = dalloc(&s->tstamp, (size_t)n * kSmallPhases)) || (rc = dalloc(&s->ls, 1)) ||
       (rc = dalloc(&s->d_degs, (size_t)opts->max_it + 2)) || (rc = dalloc(&s->d_lam_max0, n)) ||
       (rc = dalloc(&s->d_fallback, n)) || (rc = dalloc(&s->d_steps, (size_t)s->mdeg + 1)) ||
-      (rc = dalloc(&s->d_ps0, n)) || (rc = dalloc(&s->d_ferr, 1)) || (rc = dalloc(&s->d_plan, pass_plan_ints(n))))
+      (rc = dalloc(&s->d_ps0, n)) || (rc = dalloc(&s->d_ferr, 1)))
     return fail(rc);
   if (cudaMemset(s->d_ferr, 0, sizeof(int)) != cudaSuccess) return fail(LAPH_ECUDA);
   // the default filter runs a whole pass as one kernel per extent where the batch is small
   if (s->fvariant == 1 && s->kb <= 64)
     if (int e = pass_layout(s->hd, opts->link_prec == LAPH_LINKS_BF16, &s->pass)) return fail(e);
+  if (!s->pass.empty())
+    if (int e = dalloc(&s->d_plan, pass_plan_ints(n))) return fail(e);
   if (opts->link_prec == LAPH_LINKS_BF16) {
     if ((rc = dalloc(reinterpret_cast<float2**>(&s->Ubf), (size_t)o_uf))) return fail(rc);  // 4 B per element
   } else {
@@ -418,7 +420,7 @@ int laph_solver_set_links(laph_solver* s, int i, const double* links, int layout
     // device-side reorder to site-minor order through a host-free path:
     // copy to the scratch and transpose with a small kernel
     LAPH_TRY(links_to_soa_device(links, layout, d.V3, dst, s->st));
-  } else if (layout == LAPH_LAYOUT_ROWMAJOR || layout == LAPH_LAYOUT_CONF) {
+  } else if (layout == LAPH_LAYOUT_ROWMAJOR || layout == LAPH_LAYOUT_EIGEN || layout == LAPH_LAYOUT_CONF) {
     // raw copy into the staging area, reorder on the device; the finiteness
     // scan of the host links runs while the copy is in flight
     const size_t n = (layout == LAPH_LAYOUT_CONF ? 36 : 27) * (size_t)d.V3;
@@ -427,13 +429,10 @@ int laph_solver_set_links(laph_solver* s, int i, const double* links, int layout
       cudaStreamSynchronize(s->st);  // leave no copy in flight; the stored links are unchanged
       return e;
     }
-    LAPH_TRY(links_to_soa_device(reinterpret_cast<const double*>(s->stage), layout, d.V3, dst, s->st));
-  } else {
-    LAPH_TRY(check_links_finite(links, layout, d.V3, "laph_solver_set_links"));
-    std::vector<double2> soa(27 * (size_t)d.V3);
-    LAPH_TRY(links_to_soa(links, layout, d.V3, soa.data()));
-    LAPH_CUDA_TRY(cudaMemcpyAsync(dst, soa.data(), soa.size() * sizeof(double2), cudaMemcpyHostToDevice, s->st));
+    LAPH_TRY(links_reorder(s->stage, layout, d.V3, dst, true, s->st));
     LAPH_CUDA_TRY(cudaStreamSynchronize(s->st));
+  } else {
+    return check_links_finite(links, layout, d.V3, "laph_solver_set_links");  // unknown layout
   }
   s->links_set[i] = 1;
   return LAPH_OK;
@@ -584,11 +583,12 @@ static int solve_setup(laph_solver* s, bool device_loop, long long* nlaunch_out)
     for (int i = 0; i < s->np;) {
       int j = i;
       while (j < s->np && s->hd[j].L == s->hd[i].L) ++j;
-      LAPH_TRY(plaquette_moments_batch(s->U64 + s->hd[i].u64, s->hd[i].L, j - i, s->plaq + 4 * (size_t)i, s->st));
+      LAPH_TRY(plaquette_moments_batch(s->U64 + s->hd[i].u64, s->hd[i].L, j - i,
+                                       reinterpret_cast<double*>(s->W + s->hd[i].blk), s->plaq + 4 * (size_t)i, s->st));
       i = j;
     }
     LAPH_TRY(features(s->d_pd, s->np, s->U64, s->plaq, s->W, s->feats, s->bound, s->st));
-    nlaunch += 2;
+    nlaunch += 3;
     if (o.window == LAPH_WINDOW_MLP) {
       const double margin = o.window_margin > 0.0 ? o.window_margin : kWindowMargin;
       LAPH_TRY(window_infer(s->d_pd, s->d_ps, s->np, s->feats, s->model, s->mwork, s->bound, s->wdeg, margin,
