@@ -176,8 +176,8 @@ int laph_set_links(laph_ctx* c, const double* links, int layout) {
     return LAPH_EINVAL;
   }
   // The spatial links go through the two halves of the pinned staging buffer: while one half's copy is in flight the
-  // host threads check and pack the next sites into the other (a single-threaded reorder of the whole timeslice and a
-  // pageable copy took 1.9 ms at 24^3; with get_links, smearing and plaquette the set-up is 5.4 -> 0.54 ms).  The reorder on the device runs last, so links with a
+  // host threads check and pack the next sites into the other (against single-threaded reorders and pageable copies here
+  // and in laph_get_links, a 24^3 timeslice's set-up with HYP smearing and plaquette takes 0.54 instead of 5.4 ms).  The reorder on the device runs last, so links with a
   // non-finite entry leave the context's as they were.
   const int V3 = c->g.V3;
   const long long chunk = (long long)(c->half / 27);

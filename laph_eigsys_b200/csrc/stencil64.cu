@@ -94,17 +94,26 @@ int cheb64(const double2* U, int L, double lam_l, double lam_c, int deg, const d
 
 
 // ------------------------------------------- fused T_deg(B) x, one launch ---
-// The plain form's MatMult in ONE cooperative launch: every thread keeps its
-// site for the whole recurrence, so the links are read from HBM once per
-// product (forward links in 108 registers, backward links U_mu(s - mu) in
-// shared memory, as the block stencils keep them) instead of once per step,
-// and the deg steps are separated by a grid barrier instead of kernel
-// boundaries.  At 32^3 the whole product (links 14 MB, three vectors of
-// 1.5 MB) then runs from L2.  The T_n written inside the launch are read
-// with ld.global.cg (L2, never a stale L1 line); only x, read-only for the
-// launch, goes through the non-coherent path.  Used when one site per thread
-// fits the device's co-resident CTAs (up to 296 CTAs of 128 sites on a
-// B200: L <= 33); otherwise a grid-stride variant reads the links per step.
+// The plain form's MatMult in ONE launch: the deg steps are separated by a barrier
+// among the launch's CTAs instead of kernel boundaries, and where one site per
+// thread fits the chip every thread keeps its site for the whole recurrence, so
+// the links are read from HBM once per product.  At 32^3 the whole product (links
+// 14 MB, three vectors of 1.5 MB) then runs from L2.
+//
+// A step is a chain: neighbour values from L2 (written by other SMs the step
+// before), 216 FP64 complex FMAs a site (64 FMAs per SM and clock: 0.8 us for 224
+// sites), the store, the barrier.  So:
+//  - the CTAs are as many as SMs and as even as whole warps allow (147 of 224 sites
+//    at 32^3, 144 of 96 at 24^3), not 128 sites each on a part of the SMs;
+//  - the T_n are read with plain loads, so that the three colours of a 48-byte
+//    site vector share the sectors L1 fetched (reads from L2 only fetch each
+//    32-byte sector twice); the barrier's acquire keeps L1 coherent;
+//  - a lattice of at most 2048 sites is one cluster of 16 CTAs, whose barrier is
+//    the hardware's (about 0.5 us against 1.3 us through a counter in L2); at 16^3
+//    it would be 256 sites per SM, 44.5 us against 39.4 us for 128 CTAs.
+// us per product (deg 8 at 8^3, else 12), before -> now: 8^3 43.4 -> 22.3, 12^3
+// 62.5 -> 35.2, 16^3 62.5 -> 39.4, 24^3 63.9 -> 42.0, 32^3 70.4 -> 49.9, 36^3
+// 118.8 -> 98, 48^3 165.7 -> 133.
 
 // Grid barrier with a bounded wait, one atomic per CTA and arrival: every CTA
 // adds 1 to the counter except CTA 0, which adds 2^31 - (nblk - 1), so the
@@ -149,97 +158,159 @@ __device__ __forceinline__ bool grid_barrier(GridBar* b, unsigned nblk, int* her
   return s_ok != 0;
 }
 
-constexpr int kFusedSmem = 27 * 128 * (int)sizeof(double2);
+constexpr int kFusedMax = 256;  // sites of a CTA at most (resident form)
+constexpr int kFusedCluster = 16, kClusterSites = 128;  // CTAs of the one-cluster form, and sites of each at most
+constexpr int fused_smem(int ns) { return 36 * ns * (int)sizeof(double2); }
 
-template <bool RESIDENT>
-__global__ void __launch_bounds__(128, 2)
-    k_cheb64_fused(const double2* __restrict__ U, Lat g, const double2* __restrict__ x, double2* y, double2* t0,
-                   double2* t1, int deg, double c, double a, GridBar* bar, int* herr) {
-  extern __shared__ double2 s_ub[];  // [27][128] backward links (RESIDENT only)
-  double2 (*sUb)[128] = reinterpret_cast<double2 (*)[128]>(s_ub);
-  const unsigned nblk = gridDim.x;
+// y = ch hop + cd x - z for one site's three colours
+__device__ __forceinline__ double2 cheb_combine(double ch, double2 hop, double cd, double2 x, double2 z) {
+  return make_double2(ch * hop.x + cd * x.x - z.x, ch * hop.y + cd * x.y - z.y);
+}
+
+// One site per thread for the whole recurrence.  The forward links of two directions stay in 72 registers, the other
+// nine elements and the 27 backward ones in shared memory; the site's own T_{n-1} and T_{n-2} are carried in
+// registers, so a step loads only the 18 neighbour values, all in flight at once (with the third direction in registers
+// too and T_{n-1}, T_{n-2} loaded, 32^3 took 63.4 us: the loads of a step came in several rounds).
+template <bool CLUSTER>
+__global__ void __launch_bounds__(kFusedMax, 1)
+    k_cheb64_resident(const double2* __restrict__ U, Lat g, const double2* x, double2* y, double2* t0, double2* t1,
+                      int deg, double c, double a, GridBar* bar, int* herr) {
+  extern __shared__ double2 s_lk[];  // [27 + 9][blockDim.x]
+  const int nt = blockDim.x;
+  double2* sU = s_lk + threadIdx.x;
   // T_n lives in buffer (2 - (deg - n)) mod 3 of {t0, t1, y}: T_deg lands in y
   auto buf = [=](int n) {
     const int i = (((2 - (deg - n)) % 3) + 3) % 3;
     return i == 0 ? t0 : (i == 1 ? t1 : y);
   };
-  const double cd = a - 6.0 * c;
-  int s = blockIdx.x * 128 + threadIdx.x;
-  double2 uf[3][9];
+  const int s = blockIdx.x * nt + threadIdx.x;
+  const bool valid = s < g.V3;
+  double2 uf[2][9], own[3], old[3];
   int up[3], dn[3];
-  if (RESIDENT) {
-    if (s < g.V3) {
-      int sx, sy, sz;
-      site_xyz(g, s, sx, sy, sz);
+  if (valid) {
+    int sx, sy, sz;
+    site_xyz(g, s, sx, sy, sz);
 #pragma unroll
-      for (int mu = 0; mu < 3; ++mu) {
-        up[mu] = nb_up(g, sx, sy, sz, mu);
-        dn[mu] = nb_dn(g, sx, sy, sz, mu);
+    for (int mu = 0; mu < 3; ++mu) {
+      up[mu] = 3 * nb_up(g, sx, sy, sz, mu);
+      dn[mu] = 3 * nb_dn(g, sx, sy, sz, mu);
 #pragma unroll
-        for (int e = 0; e < 9; ++e) {
-          uf[mu][e] = __ldg(U + (size_t)(mu * 9 + e) * g.V3 + s);
-          sUb[mu * 9 + e][threadIdx.x] = __ldg(U + (size_t)(mu * 9 + e) * g.V3 + dn[mu]);
-        }
+      for (int e = 0; e < 9; ++e) {
+        const double2 f = __ldg(U + (size_t)(mu * 9 + e) * g.V3 + s);
+        if (mu < 2) uf[mu < 2 ? mu : 0][e] = f;
+        else sU[(27 + e) * nt] = f;
+        sU[(mu * 9 + e) * nt] = __ldg(U + (size_t)(mu * 9 + e) * g.V3 + dn[mu] / 3);
       }
     }
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      own[b] = __ldg(x + 3 * (size_t)s + b);
+      old[b] = make_double2(0.0, 0.0);
+    }
   }
+  for (int n = 1; n <= deg; ++n) {
+    if (valid) {
+      const double2* X = n == 1 ? x : buf(n - 1);
+      const double ch = n == 1 ? c : 2.0 * c, cd = n == 1 ? a - 6.0 * c : 2.0 * (a - 6.0 * c);
+      double2 xu[3][3], xd[3][3];
+#pragma unroll
+      for (int mu = 0; mu < 3; ++mu)
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+          xu[mu][b] = X[up[mu] + b];
+          xd[mu][b] = X[dn[mu] + b];
+        }
+      double2 acc[3] = {make_double2(0, 0), make_double2(0, 0), make_double2(0, 0)};
+#pragma unroll
+      for (int mu = 0; mu < 3; ++mu)
+#pragma unroll
+        for (int aa = 0; aa < 3; ++aa)
+#pragma unroll
+          for (int b = 0; b < 3; ++b) {
+            cfma(acc[aa], mu < 2 ? uf[mu < 2 ? mu : 0][3 * aa + b] : sU[(27 + 3 * aa + b) * nt], xu[mu][b]);
+            cfmac(acc[aa], sU[(mu * 9 + 3 * b + aa) * nt], xd[mu][b]);
+          }
+      double2* Y = buf(n);
+#pragma unroll
+      for (int b = 0; b < 3; ++b) {
+        const double2 r = cheb_combine(ch, acc[b], cd, own[b], old[b]);
+        old[b] = own[b];
+        own[b] = r;
+        Y[3 * (size_t)s + b] = r;
+      }
+    }
+    if (n == deg) break;
+    if (CLUSTER) {
+      // release / acquire over the cluster's CTAs, in hardware
+      asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    } else if (!grid_barrier(bar, gridDim.x, herr)) {
+      return;
+    }
+  }
+}
+
+// The same with more sites than resident threads: grid-stride, the links read per step.
+__global__ void __launch_bounds__(128, 2)
+    k_cheb64_stride(const double2* __restrict__ U, Lat g, const double2* x, double2* y, double2* t0, double2* t1,
+                    int deg, double c, double a, GridBar* bar, int* herr) {
+  auto buf = [=](int n) {
+    const int i = (((2 - (deg - n)) % 3) + 3) % 3;
+    return i == 0 ? t0 : (i == 1 ? t1 : y);
+  };
   for (int n = 1; n <= deg; ++n) {
     const double2* X = n == 1 ? x : buf(n - 1);
     const double2* Z = n == 2 ? x : (n > 2 ? buf(n - 2) : nullptr);
     double2* Y = buf(n);
-    const double ch = n == 1 ? c : 2.0 * c, cdiag = n == 1 ? cd : 2.0 * cd;
-    for (int si = s; si < g.V3; si += (RESIDENT ? g.V3 : (int)nblk * 128)) {
-      if (!RESIDENT) {
-        int sx, sy, sz;
-        site_xyz(g, si, sx, sy, sz);
-#pragma unroll
-        for (int mu = 0; mu < 3; ++mu) {
-          up[mu] = nb_up(g, sx, sy, sz, mu);
-          dn[mu] = nb_dn(g, sx, sy, sz, mu);
-        }
-      }
+    const double ch = n == 1 ? c : 2.0 * c, cd = n == 1 ? a - 6.0 * c : 2.0 * (a - 6.0 * c);
+    for (int s = blockIdx.x * 128 + threadIdx.x; s < g.V3; s += gridDim.x * 128) {
+      int sx, sy, sz;
+      site_xyz(g, s, sx, sy, sz);
       double2 acc[3] = {make_double2(0, 0), make_double2(0, 0), make_double2(0, 0)};
 #pragma unroll
       for (int mu = 0; mu < 3; ++mu) {
+        const int up = nb_up(g, sx, sy, sz, mu), dn = nb_dn(g, sx, sy, sz, mu);
         double2 xu[3], xd[3];
 #pragma unroll
         for (int b = 0; b < 3; ++b) {
-          xu[b] = n == 1 ? __ldg(X + 3 * (size_t)up[mu] + b) : __ldcg(X + 3 * (size_t)up[mu] + b);
-          xd[b] = n == 1 ? __ldg(X + 3 * (size_t)dn[mu] + b) : __ldcg(X + 3 * (size_t)dn[mu] + b);
+          xu[b] = X[3 * (size_t)up + b];
+          xd[b] = X[3 * (size_t)dn + b];
         }
 #pragma unroll
         for (int aa = 0; aa < 3; ++aa)
 #pragma unroll
           for (int b = 0; b < 3; ++b) {
-            if (RESIDENT) {
-              cfma(acc[aa], uf[mu][3 * aa + b], xu[b]);
-              cfmac(acc[aa], sUb[mu * 9 + 3 * b + aa][threadIdx.x], xd[b]);
-            } else {
-              cfma(acc[aa], __ldg(U + (size_t)(mu * 9 + 3 * aa + b) * g.V3 + si), xu[b]);
-              cfmac(acc[aa], __ldg(U + (size_t)(mu * 9 + 3 * b + aa) * g.V3 + dn[mu]), xd[b]);
-            }
+            cfma(acc[aa], __ldg(U + (size_t)(mu * 9 + 3 * aa + b) * g.V3 + s), xu[b]);
+            cfmac(acc[aa], __ldg(U + (size_t)(mu * 9 + 3 * b + aa) * g.V3 + dn), xd[b]);
           }
       }
 #pragma unroll
-      for (int aa = 0; aa < 3; ++aa) {
-        const double2 xs = n == 1 ? __ldg(X + 3 * (size_t)si + aa) : __ldcg(X + 3 * (size_t)si + aa);
-        double2 r = make_double2(ch * acc[aa].x + cdiag * xs.x, ch * acc[aa].y + cdiag * xs.y);
-        if (Z) {
-          const double2 zz = n == 2 ? __ldg(Z + 3 * (size_t)si + aa) : __ldcg(Z + 3 * (size_t)si + aa);
-          r.x -= zz.x;
-          r.y -= zz.y;
-        }
-        __stcg(Y + 3 * (size_t)si + aa, r);
-      }
+      for (int aa = 0; aa < 3; ++aa)
+        Y[3 * (size_t)s + aa] = cheb_combine(ch, acc[aa], cd, X[3 * (size_t)s + aa],
+                                             Z ? Z[3 * (size_t)s + aa] : make_double2(0.0, 0.0));
     }
-    if (n < deg && !grid_barrier(bar, nblk, herr)) return;
+    if (n < deg && !grid_barrier(bar, gridDim.x, herr)) return;
   }
 }
 
 namespace {
 struct FusedOcc {
-  int sms = 0, res = 0, nonres = 0;
+  int sms = 0, nonres = 0, clusters = 0;  // SMs, grid-stride CTAs per SM, co-resident 16-CTA clusters
 };
+cudaLaunchConfig_t cluster_config(int ns, cudaStream_t st) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(kFusedCluster);
+  cfg.blockDim = dim3(ns);
+  cfg.dynamicSmemBytes = fused_smem(ns);
+  cfg.stream = st;
+  return cfg;
+}
+cudaLaunchAttribute cluster_attribute() {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = kFusedCluster;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  return at;
+}
 std::mutex g_fused_mu;
 FusedOcc g_fused_occ[64];
 
@@ -253,11 +324,21 @@ int fused_occupancy(FusedOcc* out) {
   std::lock_guard<std::mutex> lk(g_fused_mu);
   FusedOcc& o = g_fused_occ[dev];
   if (o.sms == 0) {
-    LAPH_CUDA_TRY(cudaFuncSetAttribute(k_cheb64_fused<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       kFusedSmem));
+    LAPH_CUDA_TRY(cudaFuncSetAttribute(k_cheb64_resident<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       fused_smem(kFusedMax)));
+    LAPH_CUDA_TRY(cudaFuncSetAttribute(k_cheb64_resident<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       fused_smem(kClusterSites)));
+    LAPH_CUDA_TRY(cudaFuncSetAttribute(k_cheb64_resident<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchConfig_t cfg = cluster_config(kClusterSites, nullptr);
+    cudaLaunchAttribute at = cluster_attribute();
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&o.clusters, k_cheb64_resident<true>, &cfg) != cudaSuccess) {
+      cudaGetLastError();  // no cluster of 16 on this device: the grid form serves small lattices too
+      o.clusters = 0;
+    }
+    LAPH_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o.nonres, k_cheb64_stride, 128, 0));
     LAPH_CUDA_TRY(cudaDeviceGetAttribute(&o.sms, cudaDevAttrMultiProcessorCount, dev));
-    LAPH_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o.res, k_cheb64_fused<true>, 128, kFusedSmem));
-    LAPH_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o.nonres, k_cheb64_fused<false>, 128, 0));
   }
   *out = o;
   return LAPH_OK;
@@ -272,8 +353,18 @@ int cheb64_fused(const double2* U, int L, double lam_l, double lam_c, int deg, c
   if (deg <= 1) return hop64(U, L, x, nullptr, y, ld, 1, c, a - 6.0 * c, 0.0, st);
   FusedOcc o;
   LAPH_TRY(fused_occupancy(&o));
-  const int need = (int)ceil_div(g.V3, 128);
-  const bool resident = need <= o.res * o.sms;
+  if (g.V3 <= kFusedCluster * kClusterSites && o.clusters > 0) {
+    cudaLaunchConfig_t cfg = cluster_config((int)ceil_div(ceil_div(g.V3, kFusedCluster), 32) * 32, st);
+    cudaLaunchAttribute at = cluster_attribute();
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    LAPH_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_cheb64_resident<true>, U, g, x, y, tmp, tmp + ld, deg, c, a, bar, herr));
+    return LAPH_OK;
+  }
+  // one CTA per SM, whole warps, as even as that allows; a lattice beyond 256 sites per SM goes grid-stride
+  const int ns = (int)ceil_div(ceil_div(g.V3, o.sms), 32) * 32;
+  const bool resident = ns <= kFusedMax;
+  const int need = (int)ceil_div(g.V3, resident ? ns : 128);
   const int grid = resident ? need : std::max(1, std::min(need, o.nonres * o.sms));
   if (grid < 1 || (!resident && o.nonres < 1)) {
     set_error("cheb64_fused: no co-resident grid for L = %d", L);
@@ -287,10 +378,10 @@ int cheb64_fused(const double2* U, int L, double lam_l, double lam_c, int deg, c
   void* args[] = {(void*)&U, (void*)&gg, (void*)&x, (void*)&y, (void*)&t0, (void*)&t1, (void*)&deg, (void*)&c,
                   (void*)&a, (void*)&bar, (void*)&herr};
   if (resident)
-    LAPH_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_cheb64_fused<true>, dim3(grid), dim3(128), args,
-                                              kFusedSmem, st));
+    LAPH_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_cheb64_resident<false>, dim3(grid), dim3(ns), args,
+                                              fused_smem(ns), st));
   else
-    LAPH_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_cheb64_fused<false>, dim3(grid), dim3(128), args, 0, st));
+    LAPH_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_cheb64_stride, dim3(grid), dim3(128), args, 0, st));
   return LAPH_OK;
 }
 
