@@ -566,19 +566,18 @@ __global__ void __launch_bounds__(128) k_residual64(const ProbDesc* __restrict__
   if (threadIdx.x == 0) rpart[d.rp + (size_t)st * d.k + j] = red[0] + red[1] + red[2] + red[3];
 }
 
-// The same residual laid out like the FP64 block stencil A W: CTA = 128 sites x
-// a block of kColsFP64 columns, the site's forward links in registers and its
-// backward links in shared memory, read once per column block instead of
-// once per (site, column).  Each thread leaves |r|^2 of its site and column in
-// shared memory (FP32: one site's share of a norm needs no more); after the
-// column loop the CTA reduces the 128 sites of every column in a fixed order
-// (FP64 sums) into the same per-tile partials as the kernel above, so the
-// column loop carries no per-column reduction.
-constexpr int kResidSmem = kStencil64Smem + kColsFP64 * kSites64 * (int)sizeof(float);
+// The same residual laid out like the FP64 block stencil A W
+// (stencil64cols.cuh): CTA = 128 sites x a block of cols columns, NC per thread
+// and trip.  Each thread leaves |r|^2 of its site and columns in shared memory
+// (FP32: one site's share of a norm needs no more), and one warp sums the 128
+// sites of the trip's columns in a fixed order (FP64) into the same per-tile
+// partials as the kernel above while the others load the next trip.
+constexpr int kResidSmem = kStencil64Smem + kTrip64 * kSites64 * (int)sizeof(float);
 
-__global__ void __launch_bounds__(kSites64, 3)
+template <int NC>
+__global__ void __launch_bounds__(kThreads64, 2)
     k_residual64_cols(const ProbDesc* __restrict__ pd, const ProbState* __restrict__ ps, const int* __restrict__ start,
-                      int np, const double2* __restrict__ U64, const double2* __restrict__ Vp,
+                      int np, int cols, const double2* __restrict__ U64, const double2* __restrict__ Vp,
                       const double* __restrict__ theta, float2* __restrict__ Sp, double* __restrict__ rpart) {
   const int p = find_prob(start, np, blockIdx.x);
   if (!ps[p].active) return;
@@ -587,15 +586,16 @@ __global__ void __launch_bounds__(kSites64, 3)
   const int t = blockIdx.x - start[p];
   const int st = t % nst, cb = t / nst;
   const int c0 = ps[p].c0;
-  const int j0 = cb * kColsFP64, j1 = min(d.k, j0 + kColsFP64);
+  const int j0 = cb * cols, j1 = min(d.k, j0 + cols);
   if (j1 <= c0) return;  // frozen columns: their residual partials stand
   const int jstart = max(j0, c0);
+  const int i = threadIdx.x % kSites64, grp = threadIdx.x / kSites64;
   // threads past the last site compute the last site again and write nothing
-  const bool valid = st * kSites64 + (int)threadIdx.x < d.V3;
-  const int s = min(st * kSites64 + (int)threadIdx.x, d.V3 - 1);
+  const bool valid = st * kSites64 + i < d.V3;
+  const int s = min(st * kSites64 + i, d.V3 - 1);
   extern __shared__ double2 s64[];
-  double2 (*sUb)[kSites64] = reinterpret_cast<double2 (*)[kSites64]>(s64);
-  float (*sPart)[kSites64] = reinterpret_cast<float (*)[kSites64]>(s64 + 27 * kSites64);
+  double2 (*sU)[kSites64] = reinterpret_cast<double2 (*)[kSites64]>(s64);
+  float (*sPart)[kSites64] = reinterpret_cast<float (*)[kSites64]>(s64 + 54 * kSites64);
   const Lat g{d.L, d.L * d.L, d.V3};
   int up[3], dn[3], sx, sy, sz;
   site_xyz(g, s, sx, sy, sz);
@@ -604,36 +604,56 @@ __global__ void __launch_bounds__(kSites64, 3)
     up[mu] = nb_up(g, sx, sy, sz, mu);
     dn[mu] = nb_dn(g, sx, sy, sz, mu);
   }
-  Links64 l;
-  load_links64(U64 + d.u64, g, s, dn, l, sUb);
+  load_links64(U64 + d.u64, g, s, dn, sU, i, grp);
+  __syncthreads();
   const double sc = -2.0 * ps[p].c_hop;
 #pragma unroll 1
-  for (int j = jstart; j < j1; ++j) {
-    const size_t col = (size_t)d.blk + (size_t)j * d.dim;
-    const double2* x = Vp + col;
-    double2 acc[3];
-    hop64_col(l, sUb, d.V3, up, dn, x, acc);
-    const double th = __ldg(theta + d.kv + LAPH_IX(j, d.k));
-    double r2 = 0.0;
+  for (int jb = jstart; jb < j1; jb += kGroups64 * NC) {
+    const int j = jb + grp * NC;
+    float part[NC];
+    if (j < j1) {  // uniform over the group
+      const size_t col = (size_t)d.blk + (size_t)j * d.dim;
+      const double2* x = Vp + col;
+      int co[NC];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      const double2 xs = __ldg(x + (size_t)a * d.V3 + s);
-      const double2 r = make_double2((6.0 - th) * xs.x - acc[a].x, (6.0 - th) * xs.y - acc[a].y);
-      r2 += r.x * r.x + r.y * r.y;
-      if (valid) Sp[col + (size_t)a * d.V3 + s] = make_float2((float)(sc * r.x), (float)(sc * r.y));
+      for (int c = 0; c < NC; ++c) co[c] = min(c, j1 - 1 - j) * (int)d.dim;
+      double2 acc[NC][3];
+      if (i == 0)  // the group's next columns into L2
+        for (int c = kGroups64 * NC; c < min((kGroups64 + 1) * NC, j1 - j); ++c)
+          prefetch64(x + (size_t)c * d.dim, d.V3, st * kSites64);
+      hop64_cols<NC>(sU, i, d.V3, up, dn, x, co, acc);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const double th = __ldg(theta + d.kv + LAPH_IX(min(j + c, j1 - 1), d.k));
+        double r2 = 0.0;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          const double2 xs = __ldg(x + co[c] + a * d.V3 + s);
+          const double2 r = make_double2((6.0 - th) * xs.x - acc[c][a].x, (6.0 - th) * xs.y - acc[c][a].y);
+          r2 += r.x * r.x + r.y * r.y;
+          if (valid && j + c < j1) Sp[col + co[c] + a * d.V3 + s] = make_float2((float)(sc * r.x), (float)(sc * r.y));
+        }
+        part[c] = valid ? (float)r2 : 0.f;
+      }
     }
-    sPart[LAPH_IX(j - j0, kColsFP64)][threadIdx.x] = valid ? (float)r2 : 0.f;
-  }
-  __syncthreads();
-  // column c = tid / 4 summed by 4 threads over 32 sites each, then across them
-  const int c = threadIdx.x >> 2, q = threadIdx.x & 3;
-  double sum = 0.0;
-  if (j0 + c >= jstart && j0 + c < j1)
+    __syncthreads();  // the sums of the trip before are done
+    if (j < j1)
+#pragma unroll
+      for (int c = 0; c < NC; ++c) sPart[grp * NC + c][i] = part[c];
+    __syncthreads();
+    // column c = tid / 4 summed by 4 threads over 32 sites each, then across them
+    if (threadIdx.x < 32) {
+      const int c = threadIdx.x >> 2, q = threadIdx.x & 3;
+      const bool live = c < kGroups64 * NC && jb + c < j1;
+      double sum = 0.0;
+      if (live)
 #pragma unroll 8
-    for (int i = 0; i < kSites64 / 4; ++i) sum += (double)sPart[c][q * (kSites64 / 4) + i];
-  sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-  sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-  if (q == 0 && j0 + c >= jstart && j0 + c < j1) rpart[d.rp + (size_t)st * d.k + j0 + c] = sum;
+        for (int e = 0; e < kSites64 / 4; ++e) sum += (double)sPart[c][q * (kSites64 / 4) + e];
+      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+      if (q == 0 && live) rpart[d.rp + (size_t)st * d.k + jb + c] = sum;
+    }
+  }
 }
 
 // ------------------------------------------------------- residuals/conv ----
@@ -777,7 +797,9 @@ int dense_init() {
   LAPH_CUDA_TRY(cudaFuncSetAttribute(k_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, kGramSmem));
   LAPH_CUDA_TRY(cudaFuncSetAttribute(k_gram_split, cudaFuncAttributeMaxDynamicSharedMemorySize, kGramSplitSmem));
   LAPH_CUDA_TRY(cudaFuncSetAttribute(k_rotate, cudaFuncAttributeMaxDynamicSharedMemorySize, kRotSmem));
-  LAPH_CUDA_TRY(cudaFuncSetAttribute(k_residual64_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, kResidSmem));
+  LAPH_CUDA_TRY(cudaFuncSetAttribute(k_residual64_cols<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kResidSmem));
+  LAPH_CUDA_TRY(cudaFuncSetAttribute(k_residual64_cols<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kResidSmem));
+  LAPH_CUDA_TRY(cudaFuncSetAttribute(k_residual64_cols<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kResidSmem));
   LAPH_TRY(neglap64_init());
   return small_init();
 }
@@ -814,9 +836,14 @@ int residual64(const ProbDesc* pd, const ProbState* ps, const int* start, int np
   LAPH_CUDA_TRY(cudaGetLastError());
   return LAPH_OK;
 }
-int residual64_cols(const ProbDesc* pd, const ProbState* ps, const int* start, int np, int nblk, const double2* U64,
-                    const double2* V, const double* theta, float2* S, double* rpart, cudaStream_t st) {
-  k_residual64_cols<<<nblk, kSites64, kResidSmem, st>>>(pd, ps, start, np, U64, V, theta, S, rpart);
+int residual64_cols(const ProbDesc* pd, const ProbState* ps, const int* start, int np, int nblk, int cols,
+                    const double2* U64, const double2* V, const double* theta, float2* S, double* rpart, cudaStream_t st) {
+  if (cols >= 4 * kGroups64)
+    k_residual64_cols<4><<<nblk, kThreads64, kResidSmem, st>>>(pd, ps, start, np, cols, U64, V, theta, S, rpart);
+  else if (cols >= 2 * kGroups64)
+    k_residual64_cols<2><<<nblk, kThreads64, kResidSmem, st>>>(pd, ps, start, np, cols, U64, V, theta, S, rpart);
+  else
+    k_residual64_cols<1><<<nblk, kThreads64, kResidSmem, st>>>(pd, ps, start, np, cols, U64, V, theta, S, rpart);
   LAPH_CUDA_TRY(cudaGetLastError());
   return LAPH_OK;
 }

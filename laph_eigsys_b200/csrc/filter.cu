@@ -389,20 +389,23 @@ __global__ void k_direct_start(const ProbDesc* __restrict__ pd, const ProbState*
 
 // ------------------------------------------------ FP64 block stencil: A W --
 // Y_j = (-Delta) W_j = 6 W_j - hop(W_j), FP64; CTA = 128 sites x a block of
-// kColsFP64 columns (stencil64cols.cuh).
-__global__ void __launch_bounds__(128, 3) k_neglap64_batch(const ProbDesc* __restrict__ pd, const ProbState* __restrict__ ps,
-                                                        const int* __restrict__ start, int np,
-                                                        const double2* __restrict__ U64, const double2* __restrict__ Wp,
-                                                        double2* __restrict__ Yp) {
+// cols columns, NC per thread and trip (stencil64cols.cuh).
+template <int NC>
+__global__ void __launch_bounds__(kThreads64, 2)
+    k_neglap64_batch(const ProbDesc* __restrict__ pd, const ProbState* __restrict__ ps, const int* __restrict__ start,
+                     int np, int cols, const double2* __restrict__ U64, const double2* __restrict__ Wp,
+                     double2* __restrict__ Yp) {
   const int p = find_prob(start, np, blockIdx.x);
   if (!ps[p].active) return;
   const ProbDesc d = pd[p];
   const int nst = (d.V3 + kSites64 - 1) / kSites64;
   const int t = blockIdx.x - start[p];
   const int st = t % nst, cb = t / nst;
-  if ((cb + 1) * kColsFP64 <= ps[p].c0) return;  // frozen columns: Y not needed
-  const int s = st * kSites64 + threadIdx.x;
-  if (s >= d.V3) return;
+  if ((cb + 1) * cols <= ps[p].c0) return;  // frozen columns: Y not needed
+  const int i = threadIdx.x % kSites64, grp = threadIdx.x / kSites64;
+  // threads past the last site compute the last site again and write nothing
+  const bool valid = st * kSites64 + i < d.V3;
+  const int s = min(st * kSites64 + i, d.V3 - 1);
   const Lat g{d.L, d.L * d.L, d.V3};
   int sx, sy, sz, up[3], dn[3];
   site_xyz(g, s, sx, sy, sz);
@@ -412,20 +415,30 @@ __global__ void __launch_bounds__(128, 3) k_neglap64_batch(const ProbDesc* __res
     dn[mu] = nb_dn(g, sx, sy, sz, mu);
   }
   extern __shared__ double2 s64[];
-  double2 (*sUb)[kSites64] = reinterpret_cast<double2 (*)[kSites64]>(s64);
-  Links64 l;
-  load_links64(U64 + d.u64, g, s, dn, l, sUb);
-  const int j1 = min(d.k, (cb + 1) * kColsFP64);
+  double2 (*sU)[kSites64] = reinterpret_cast<double2 (*)[kSites64]>(s64);
+  const int j0 = cb * cols, j1 = min(d.k, j0 + cols);
+  load_links64(U64 + d.u64, g, s, dn, sU, i, grp);
+  __syncthreads();
 #pragma unroll 1
-  for (int j = cb * kColsFP64; j < j1; ++j) {
+  for (int j = j0 + grp * NC; j < j1; j += kGroups64 * NC) {
     const size_t col = (size_t)d.blk + (size_t)j * d.dim;
     const double2* x = Wp + col;
-    double2 acc[3];
-    hop64_col(l, sUb, d.V3, up, dn, x, acc);
+    int co[NC];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      const double2 xs = __ldg(x + (size_t)a * d.V3 + s);
-      Yp[col + (size_t)a * d.V3 + s] = make_double2(6.0 * xs.x - acc[a].x, 6.0 * xs.y - acc[a].y);
+    for (int c = 0; c < NC; ++c) co[c] = min(c, j1 - 1 - j) * (int)d.dim;
+    double2 acc[NC][3];
+    if (i == 0)  // the group's next columns into L2
+      for (int c = kGroups64 * NC; c < min((kGroups64 + 1) * NC, j1 - j); ++c)
+        prefetch64(x + (size_t)c * d.dim, d.V3, st * kSites64);
+    hop64_cols<NC>(sU, i, d.V3, up, dn, x, co, acc);
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      if (!valid || j + c >= j1) continue;
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const double2 xs = __ldg(x + co[c] + a * d.V3 + s);
+        Yp[col + co[c] + a * d.V3 + s] = make_double2(6.0 * xs.x - acc[c][a].x, 6.0 * xs.y - acc[c][a].y);
+      }
     }
   }
 }
@@ -579,13 +592,21 @@ int direct_start(const ProbDesc* pd, const ProbState* ps, const int* start, int 
 }
 
 int neglap64_init() {
-  LAPH_CUDA_TRY(cudaFuncSetAttribute(k_neglap64_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, kStencil64Smem));
+  LAPH_CUDA_TRY(cudaFuncSetAttribute(k_neglap64_batch<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStencil64Smem));
+  LAPH_CUDA_TRY(cudaFuncSetAttribute(k_neglap64_batch<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStencil64Smem));
+  LAPH_CUDA_TRY(cudaFuncSetAttribute(k_neglap64_batch<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStencil64Smem));
   return LAPH_OK;
 }
 
-int neglap64_batch(const ProbDesc* pd, const ProbState* ps, const int* start, int np, int nblk, const double2* U64,
+int neglap64_batch(const ProbDesc* pd, const ProbState* ps, const int* start, int np, int nblk, int cols,
+                   const double2* U64,
                    const double2* W, double2* Y, cudaStream_t st) {
-  k_neglap64_batch<<<nblk, kSites64, kStencil64Smem, st>>>(pd, ps, start, np, U64, W, Y);
+  if (cols >= 4 * kGroups64)
+    k_neglap64_batch<4><<<nblk, kThreads64, kStencil64Smem, st>>>(pd, ps, start, np, cols, U64, W, Y);
+  else if (cols >= 2 * kGroups64)
+    k_neglap64_batch<2><<<nblk, kThreads64, kStencil64Smem, st>>>(pd, ps, start, np, cols, U64, W, Y);
+  else
+    k_neglap64_batch<1><<<nblk, kThreads64, kStencil64Smem, st>>>(pd, ps, start, np, cols, U64, W, Y);
   LAPH_CUDA_TRY(cudaGetLastError());
   return LAPH_OK;
 }

@@ -33,9 +33,9 @@ int direct_start(const ProbDesc* pd, const ProbState* ps, const int* start, int 
 int cheb_init();
 // Opt the FP64 stencil into its dynamic shared memory on the current device.
 int neglap64_init();
-// Y = (-Delta) W for every column, FP64.
-int neglap64_batch(const ProbDesc* pd, const ProbState* ps, const int* start, int np, int nblk, const double2* U64,
-                   const double2* W, double2* Y, cudaStream_t st);
+// Y = (-Delta) W for every column, FP64; CTA = 128 sites x cols columns, 2 .. 32.
+int neglap64_batch(const ProbDesc* pd, const ProbState* ps, const int* start, int np, int nblk, int cols,
+                   const double2* U64, const double2* W, double2* Y, cudaStream_t st);
 // Gaussian random start block.
 int random_block(const ProbDesc* pd, const int* start, int np, int nblk, double2* W, uint64_t seed, cudaStream_t st);
 }  // namespace laph

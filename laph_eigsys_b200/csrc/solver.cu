@@ -54,6 +54,7 @@ struct laph_solver {
   cudaStream_t st = nullptr;
   laph_solve_opts o{};
   int np = 0, mdeg = 16, kb = 32, tile = 128;
+  int cols64 = kColsFP64;  // columns per CTA of the FP64 block stencils
   int kmax = 0;                // widest block of the batch
   int fvariant = 1, lmax = 0;  // filter variant in use (opts.filter_kernel, or 1 where 3 does not apply)
   int* d_ferr = nullptr;       // set by a filter kernel whose bounded wait gave up
@@ -265,6 +266,19 @@ int laph_solver_create(laph_solver** out, const laph_problem* probs, int n, cons
   long long work = 0;
   for (int i = 0; i < n; ++i) work += (long long)probs[i].L * probs[i].L * probs[i].L * round_up(probs[i].nev + opts->guard, kGramTile);
   s->kb = opts->block > 0 ? opts->block : work < 8000000 ? 16 : 32;
+  // Columns per CTA of the FP64 stencils: 32, halved while the batch gives fewer CTAs than the device has SMs (down to 2:
+  // one per thread group).  A W, us at 32 / 16 / 8 / 4 / 2: 7^3 x 32 columns 27.5 / 16.1 / 10.0 / 6.7 / 5.5; 8^3 x 8
+  // x 32 28.3 / 16.3 / 10.5 / 9.8 / 14.4; 16^3 x 96 30.8 / 23.1 / 23.2 / 25.7 / 36.6; 24^3 x 160 98 / 104 / 112 / 134 / 201
+  auto blocks64 = [&](int cols) {
+    long long b = 0;
+    for (int i = 0; i < n; ++i) {
+      const int V3 = probs[i].L * probs[i].L * probs[i].L, k = round_up(probs[i].nev + opts->guard, kGramTile);
+      b += (long long)((V3 + kSites64 - 1) / kSites64) * ((k + cols - 1) / cols);
+    }
+    return b;
+  };
+  s->cols64 = kColsFP64;
+  while (s->cols64 > 2 && blocks64(s->cols64) < 148) s->cols64 /= 2;
   // sites per CTA of the filter; the per-thread-coefficient variant and blocks wider than 64 keep 128
   s->tile = opts->filter_tile > 0 && opts->filter_kernel >= 1 && s->kb <= 64 ? opts->filter_tile : 128;
   // the staged variant (3) needs 128-site tiles of whole z-rows inside one plane for every problem
@@ -323,7 +337,7 @@ int laph_solver_create(laph_solver** out, const laph_problem* probs, int n, cons
     const int nst = (d.V3 + 127) / 128;
     per_site.push_back(nst);
     per_filt.push_back(((d.V3 + s->tile - 1) / s->tile) * ((d.k + s->kb - 1) / s->kb));
-    per_nl.push_back(nst * ((d.k + kColsFP64 - 1) / kColsFP64));
+    per_nl.push_back(nst * ((d.k + s->cols64 - 1) / s->cols64));
     per_res.push_back(nst * d.k);
     per_gram.push_back(d.nchunk * npair);
     per_gred.push_back((2 * npair * kGramTile * kGramTile + 255) / 256);
@@ -458,7 +472,7 @@ static int residual(laph_solver* s) {
   }();
   if (kind == 0)
     return residual64(s->d_pd, s->d_ps, s->st_res, s->np, s->nb_res, s->U64, s->V, s->theta, s->S, s->rpart, s->st);
-  return residual64_cols(s->d_pd, s->d_ps, s->st_nl, s->np, s->nb_nl, s->U64, s->V, s->theta, s->S, s->rpart, s->st);
+  return residual64_cols(s->d_pd, s->d_ps, s->st_nl, s->np, s->nb_nl, s->cols64, s->U64, s->V, s->theta, s->S, s->rpart, s->st);
 }
 
 static int jacobi_sweeps(const laph_solver* s) { return s->o.jacobi_sweeps > 0 ? s->o.jacobi_sweeps : 2; }
@@ -467,7 +481,7 @@ static long long rr_launches(const laph_solver* s) { return 7 + small_launches(s
 
 static int iteration_rr(laph_solver* s, int first_iter) {
   const bool fixed = s->o.window == LAPH_WINDOW_FIXED && s->o.lam_cut > 0.0;
-  LAPH_TRY(neglap64_batch(s->d_pd, s->d_ps, s->st_nl, s->np, s->nb_nl, s->U64, s->W, s->Y, s->st));
+  LAPH_TRY(neglap64_batch(s->d_pd, s->d_ps, s->st_nl, s->np, s->nb_nl, s->cols64, s->U64, s->W, s->Y, s->st));
   LAPH_TRY(gram(s->d_pd, s->d_ps, s->st_gram, s->np, s->nb_gram, 8192, s->W, s->Y, s->gpart, s->st));
   LAPH_TRY(gram_reduce(s->d_pd, s->d_ps, s->st_gred, s->np, s->nb_gred, s->gpart, s->KK, s->st));
   LAPH_TRY(small_dense(s->d_pd, s->d_ps, s->np, s->kmax, s->KK, s->theta, s->dwork, first_iter, fixed ? 1 : 0,
