@@ -24,7 +24,7 @@
 // the rest of the chip idled.  Now the only serial chains are the Jacobi's
 // steps (shared memory of a cluster) and the Cholesky's columns; per pass at
 // n = 160, us before -> now: Cholesky 1540 -> 165, inverse 906 -> 63, projection
-// 1500 -> 43, Jacobi 6380 -> 832, C 537 -> 160.  Every element
+// 1500 -> 43, Jacobi 6380 -> 795, C 537 -> 160.  Every element
 // still sees the same operations in the same order as in the unblocked loops
 // (sums run over ascending q, updates subtract one term at a time), so the split
 // over tiles and CTAs does not change a bit of the result.
@@ -496,12 +496,29 @@ __global__ void __launch_bounds__(256) k_prod(const ProbDesc* __restrict__ pd, c
 // barrier and one CTA barrier.  The product of the rotations is not kept here:
 // they go to a log that k_apply replays.  n > kJacSmemN keeps both
 // copies in global memory (Ht and the Cholesky factor's storage), same code.
-// A step costs 1.8-3.1 us (n = 64 .. 256) where one SM took 4.3-50 us; about half
-// of it is the chain of square roots and divisions of a rotation.
+// A step costs 1.4-3.9 us (n = 64 .. 320) where one SM took 4.3-50 us; much of it is
+// the chain of square roots and divisions of a rotation.  In clusters of 8 one half
+// of the threads takes it for the angles, the other for the phases, and the test
+// for a rotation needs no square root of its own (2 sweeps, us: n = 32 115 -> 87, 64
+// 232 -> 183, 96 384 -> 336, 160 835 -> 796, 224 1616 -> 1567); in clusters of 16 the second
+// read of every pivot from its owner costs more than that (n = 320 2450 -> 2850), and one
+// thread takes both.  Clusters of 1, 2 and 4 where they hold the matrix: n = 32 89,
+// 92, 92; 64 290, 231, 206; 160 in 4 1109.
 constexpr int kJacThreads = 512;
 constexpr int kJacSmemN8 = 224, kJacSmemN16 = 320;  // largest n whose two copies fit 8 / 16 CTAs
 
 __device__ __forceinline__ int jac_shift(int pos, int n) { return pos == 0 ? 0 : (pos == n - 1 ? 1 : pos + 1); }
+
+// rr > 1e-300 and rr > 1e-18 sqrt(|app aqq|); the square root only where the squares, a factor 2 apart, do not decide
+__device__ __forceinline__ bool jac_rotates(double rr, double app, double aqq) {
+  const double m = fabs(app * aqq);
+  if (rr > 1e-120 && rr < 1e120 && m < 1e240) {
+    const double q = rr * rr;
+    if (q > 2e-36 * m) return true;
+    if (q < 0.5e-36 * m) return false;
+  }
+  return rr > 1e-300 && rr > 1e-18 * sqrt(m);
+}
 
 template <int C, bool SM>
 __global__ void __launch_bounds__(kJacThreads) k_jacobi(const ProbDesc* __restrict__ pd, ProbState* __restrict__ ps,
@@ -541,6 +558,12 @@ __global__ void __launch_bounds__(kJacThreads) k_jacobi(const ProbDesc* __restri
     }
   __syncthreads();
   cl.sync();
+  constexpr bool kSplit = C == 8;
+  const int pr = kSplit ? tid & 255 : tid;
+  const bool angle = !kSplit || tid < 256, phase = !kSplit || tid >= 256, logs = pr / PP == rk;
+  // columns of the thread's pair in either copy
+  const int pc = min(pr, half - 1);
+  const double2 *cp0 = column(0, pc), *cp1 = column(1, pc), *cq0 = column(0, n - 1 - pc), *cq1 = column(1, n - 1 - pc);
   int cur = 0, t = 0;
   for (int sweep = 0; sweep < sweeps; ++sweep) {
     double off = 0.0, dia = 0.0;
@@ -578,28 +601,30 @@ __global__ void __launch_bounds__(kJacThreads) k_jacobi(const ProbDesc* __restri
     double2* log = sweep == 0 ? v.H : v.T1;
     for (int step = 0; step < n - 1; ++step, ++t) {
       // rotation of pair r = (r, n-1-r): J (p,p)=c (p,q)=s (q,p)=-s e (q,q)=c e, e = e^{-i phi}
-      for (int r = tid; r < half; r += kJacThreads) {
-        const double2* cp = column(cur, r);
-        const double2* cq = column(cur, n - 1 - r);
-        const double2 g = cq[r];
-        const double app = cp[r].x, aqq = cq[n - 1 - r].x;
+      if (pr < half) {
+        const double2 *cp = cur ? cp1 : cp0, *cq = cur ? cq1 : cq0;
+        const double2 g = cq[pr];
+        const double app = cp[pr].x, aqq = cq[n - 1 - pr].x;
         const double rr = hypot(g.x, g.y);
-        double c = 1.0, s = 0.0;
-        double2 em = make_double2(1.0, 0.0);
-        if (rr > 1e-300 && rr > 1e-18 * sqrt(fabs(app * aqq))) {
-          em = make_double2(g.x / rr, -g.y / rr);
-          const double tau = (aqq - app) / (2.0 * rr);
-          const double tt = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
-          c = 1.0 / sqrt(1.0 + tt * tt);
-          s = tt * c;
+        const bool rot = jac_rotates(rr, app, aqq);
+        double2* o = log + 2 * ((size_t)step * half + pr);
+        if (phase) {
+          double2 em = make_double2(1.0, 0.0);
+          if (rot) em = make_double2(g.x / rr, -g.y / rr);
+          s_e[pr] = em;
+          if (logs) o[1] = em;
         }
-        s_c[r] = c;
-        s_s[r] = s;
-        s_e[r] = em;
-        if (r / PP == rk) {
-          double2* o = log + 2 * ((size_t)step * half + r);
-          o[0] = make_double2(c, s);
-          o[1] = em;
+        if (angle) {
+          double c = 1.0, s = 0.0;
+          if (rot) {
+            const double tau = (aqq - app) / (2.0 * rr);
+            const double tt = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
+            c = 1.0 / sqrt(1.0 + tt * tt);
+            s = tt * c;
+          }
+          s_c[pr] = c;
+          s_s[pr] = s;
+          if (logs) o[0] = make_double2(c, s);
         }
       }
       __syncthreads();
