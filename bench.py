@@ -532,7 +532,7 @@ def measure_matvec_fp64(cfg, batch, device, deg=12, reps=20):
     return {"workload": f"T_{deg}(B) x on one {L}^3 vector, FP64 (laph_matmult, device pointers)",
             "ms_per_matmult": ms, "bytes_per_matmult": byts, "achieved_gbs": byts / (ms / 1e3) / 1e9,
             "peak_gbs": hbm, "peak_source": src, "frac": byts / (ms / 1e3) / 1e9 / hbm,
-            "kernel": "k_cheb64_fused (one cooperative launch per product)",
+            "kernel": "k_cheb64_resident (one cooperative launch per product)",
             "timing": "CUDA events on the context's stream around each call (device time of the product and its "
                       "error-flag read), mean of the calls", "host_ms_per_matmult": host_ms}
 
