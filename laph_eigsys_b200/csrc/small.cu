@@ -24,7 +24,7 @@
 // the rest of the chip idled.  Now the only serial chains are the Jacobi's
 // steps (shared memory of a cluster) and the Cholesky's columns; per pass at
 // n = 160, us before -> now: Cholesky 1540 -> 165, inverse 906 -> 63, projection
-// 1500 -> 43, Jacobi 6380 -> 795, C 537 -> 160.  Every element
+// 1500 -> 43, Jacobi 6380 -> 772, C 537 -> 160.  Every element
 // still sees the same operations in the same order as in the unblocked loops
 // (sums run over ascending q, updates subtract one term at a time), so the split
 // over tiles and CTAs does not change a bit of the result.
@@ -497,14 +497,18 @@ __global__ void __launch_bounds__(256) k_prod(const ProbDesc* __restrict__ pd, c
 // they go to a log that k_apply replays.  n > kJacSmemN keeps both
 // copies in global memory (Ht and the Cholesky factor's storage), same code.
 // A step costs 1.4-3.9 us (n = 64 .. 320) where one SM took 4.3-50 us; much of it is
-// the chain of square roots and divisions of a rotation.  In clusters of 8 one half
-// of the threads takes it for the angles, the other for the phases, and the test
-// for a rotation needs no square root of its own (2 sweeps, us: n = 32 115 -> 87, 64
-// 232 -> 183, 96 384 -> 336, 160 835 -> 796, 224 1616 -> 1567); in clusters of 16 the second
-// read of every pivot from its owner costs more than that (n = 320 2450 -> 2850), and one
-// thread takes both.  Clusters of 1, 2 and 4 where they hold the matrix: n = 32 89,
-// 92, 92; 64 290, 231, 206; 160 in 4 1109.
+// the chain of square roots and divisions of a rotation.  The test for a rotation needs
+// no square root of its own, and up to n = 128 and in global memory (SPLIT) one half
+// of the threads takes the chain for the angles, the other for the phases.  Above, the
+// second read of every pivot from its owner costs more than that gives (n = 224 1519
+// -> 1570, 320 2380 -> 2850).  Clusters of 8 keep to 64 registers, two CTAs an SM: at
+// 121 the clusters of 16 problems do not fit the device at once (n = 96 437 -> 673 us).
+// 2 sweeps, us, before -> now, 1 or 2 problems: n = 32 115 -> 88, 128 583 -> 552, 160 835
+// -> 772, 224 1617 -> 1519, 320 2466 -> 2379, 416 5600 -> 4460; 8 of 64 232 -> 184; 16
+// of 64 257 -> 225, of 96 452 -> 437, of 128 692 -> 694, of 160 1010 -> 1001.  Clusters of
+// 1, 2 and 4 where they hold the matrix: n = 32 89, 92, 92; 64 290, 231, 206; 160 in 4 1109.
 constexpr int kJacThreads = 512;
+constexpr int kJacSplitN = 128;  // up to here angles and phases of the rotations run on separate threads
 constexpr int kJacSmemN8 = 224, kJacSmemN16 = 320;  // largest n whose two copies fit 8 / 16 CTAs
 
 __device__ __forceinline__ int jac_shift(int pos, int n) { return pos == 0 ? 0 : (pos == n - 1 ? 1 : pos + 1); }
@@ -520,8 +524,8 @@ __device__ __forceinline__ bool jac_rotates(double rr, double app, double aqq) {
   return rr > 1e-300 && rr > 1e-18 * sqrt(m);
 }
 
-template <int C, bool SM>
-__global__ void __launch_bounds__(kJacThreads) k_jacobi(const ProbDesc* __restrict__ pd, ProbState* __restrict__ ps,
+template <int C, bool SM, bool SPLIT>
+__global__ void __launch_bounds__(kJacThreads, C == 8 ? 2 : 1) k_jacobi(const ProbDesc* __restrict__ pd, ProbState* __restrict__ ps,
                                                         double2* KK, double* theta, double* dwork, int first_iter,
                                                         int fixed_cut, int sweeps, int last,
                                                         unsigned long long* tstamp) {
@@ -558,9 +562,8 @@ __global__ void __launch_bounds__(kJacThreads) k_jacobi(const ProbDesc* __restri
     }
   __syncthreads();
   cl.sync();
-  constexpr bool kSplit = C == 8;
-  const int pr = kSplit ? tid & 255 : tid;
-  const bool angle = !kSplit || tid < 256, phase = !kSplit || tid >= 256, logs = pr / PP == rk;
+  const int pr = SPLIT ? tid & 255 : tid;
+  const bool angle = !SPLIT || tid < 256, phase = !SPLIT || tid >= 256, logs = pr / PP == rk;
   // columns of the thread's pair in either copy
   const int pc = min(pr, half - 1);
   const double2 *cp0 = column(0, pc), *cp1 = column(1, pc), *cq0 = column(0, n - 1 - pc), *cq1 = column(1, n - 1 - pc);
@@ -861,7 +864,7 @@ __global__ void __launch_bounds__(256) k_lift(const ProbDesc* __restrict__ pd, c
           make_double2(-acc[a][b].x, -acc[a][b].y);
 }
 
-template <int C, bool SM>
+template <int C, bool SM, bool SPLIT>
 int launch_jacobi(const ProbDesc* pd, ProbState* ps, int np, int smem, double2* KK, double* theta, double* dwork,
                   int first_iter, int fixed_cut, int sweeps, int last, unsigned long long* tstamp, cudaStream_t st) {
   cudaLaunchConfig_t cfg{};
@@ -875,7 +878,7 @@ int launch_jacobi(const ProbDesc* pd, ProbState* ps, int np, int smem, double2* 
   at.val.clusterDim.y = at.val.clusterDim.z = 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  LAPH_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_jacobi<C, SM>, pd, ps, KK, theta, dwork, first_iter, fixed_cut, sweeps, last,
+  LAPH_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_jacobi<C, SM, SPLIT>, pd, ps, KK, theta, dwork, first_iter, fixed_cut, sweeps, last,
                                    tstamp));
   return LAPH_OK;
 }
@@ -889,11 +892,13 @@ int small_init() {
   LAPH_CUDA_TRY(cudaFuncSetAttribute(k_apply<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, apply_smem(160)));
   LAPH_CUDA_TRY(cudaFuncSetAttribute(k_apply<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, apply_smem(256)));
   LAPH_CUDA_TRY(cudaFuncSetAttribute(k_apply<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, apply_smem(512)));
-  LAPH_CUDA_TRY(cudaFuncSetAttribute(k_jacobi<8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  LAPH_CUDA_TRY(cudaFuncSetAttribute(k_jacobi<8, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     4 * kJacSplitN * kJacSplitN));
+  LAPH_CUDA_TRY(cudaFuncSetAttribute(k_jacobi<8, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      4 * kJacSmemN8 * kJacSmemN8));
-  LAPH_CUDA_TRY(cudaFuncSetAttribute(k_jacobi<16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  LAPH_CUDA_TRY(cudaFuncSetAttribute(k_jacobi<16, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      2 * kJacSmemN16 * kJacSmemN16));
-  LAPH_CUDA_TRY(cudaFuncSetAttribute(k_jacobi<16, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  LAPH_CUDA_TRY(cudaFuncSetAttribute(k_jacobi<16, true, false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   return LAPH_OK;
 }
 
@@ -920,14 +925,17 @@ int small_dense(const ProbDesc* pd, ProbState* ps, int np, int kmax, double2* KK
   const int global = kmax > kJacSmemN16, per = global ? 1 : 2;
   for (int s = 0; s < max_sweeps; s += per) {
     const int ns = std::min(per, max_sweeps - s), last = s + per >= max_sweeps;
-    if (kmax <= kJacSmemN8)
-      LAPH_TRY((launch_jacobi<8, true>(pd, ps, np, 4 * kmax * kmax, KK, theta, dwork, first_iter, fixed_cut, ns, last,
+    if (kmax <= kJacSplitN)
+      LAPH_TRY((launch_jacobi<8, true, true>(pd, ps, np, 4 * kmax * kmax, KK, theta, dwork, first_iter, fixed_cut, ns,
+                                             last, tstamp, st)));
+    else if (kmax <= kJacSmemN8)
+      LAPH_TRY((launch_jacobi<8, true, false>(pd, ps, np, 4 * kmax * kmax, KK, theta, dwork, first_iter, fixed_cut, ns, last,
                                        tstamp, st)));
     else if (!global)
-      LAPH_TRY((launch_jacobi<16, true>(pd, ps, np, 2 * kmax * kmax, KK, theta, dwork, first_iter, fixed_cut, ns, last,
+      LAPH_TRY((launch_jacobi<16, true, false>(pd, ps, np, 2 * kmax * kmax, KK, theta, dwork, first_iter, fixed_cut, ns, last,
                                         tstamp, st)));
     else
-      LAPH_TRY((launch_jacobi<8, false>(pd, ps, np, 0, KK, theta, dwork, first_iter, fixed_cut, ns, last, tstamp, st)));
+      LAPH_TRY((launch_jacobi<8, false, true>(pd, ps, np, 0, KK, theta, dwork, first_iter, fixed_cut, ns, last, tstamp, st)));
     const dim3 rows((kmax + kApplyRows - 1) / kApplyRows, np);
     auto apply = kmax <= 160 ? k_apply<5> : kmax <= 256 ? k_apply<8> : k_apply<16>;
     apply<<<rows, kApplyThreads, apply_smem(kmax), st>>>(pd, ps, KK, theta, dwork, s == 0, last, global, tstamp);
