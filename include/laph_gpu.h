@@ -206,13 +206,16 @@ typedef struct {
   int phase_fix;        /* apply fix_phase to the output eigenvectors             */
   uint64_t seed;        /* start block                                            */
   int block;            /* columns per CTA of the filter kernel, 1..512 (0: 32, or
-                           16 for a small batch); above 64 the filter runs as
-                           variant 0                                             */
+                           16 below 8e6 site-columns in the batch); above 64 the
+                           filter runs as variant 0                              */
   int filter_kernel;    /* filter variant, all with register-resident forward
                            links and L2 bulk prefetch: 0 FP64 coefficients per
                            thread; 1 FP32 coefficients staged per CTA, backward
-                           links in shared memory (default; block <= 64; a small
-                           batch runs each whole pass as one kernel); 2 as 1
+                           links in shared memory (default; block <= 64; a batch of
+                           at most 3e6 site-columns with block 0 or 16 and
+                           filter_tile 0 or 128 runs each whole pass as one
+                           kernel, which has neither; any other block or tile
+                           takes the kernels that run step by step); 2 as 1
                            with the backward links in tensor memory; 3 as 2 with
                            the vectors staged by a bulk-copy pipeline; 4 as 2 on
                            512-site bricks; 5 as 2 with each thread's next-column

@@ -158,6 +158,8 @@ int upload_prefix(const std::vector<int>& per, int** d, int* total) {
   return LAPH_OK;
 }
 
+constexpr int kSmallBlock = 16;  // columns per CTA of the filter for a small batch
+
 int round_up(int a, int b) { return (a + b - 1) / b * b; }
 
 }  // namespace
@@ -265,7 +267,7 @@ int laph_solver_create(laph_solver** out, const laph_problem* probs, int n, cons
   // 24^3 x 2 and 32^3 x 1, 160 columns: 4.1e10 against 3.9e10 site-columns a second, 32^3 x 2: 4.6e10 either way)
   long long work = 0;
   for (int i = 0; i < n; ++i) work += (long long)probs[i].L * probs[i].L * probs[i].L * round_up(probs[i].nev + opts->guard, kGramTile);
-  s->kb = opts->block > 0 ? opts->block : work < 8000000 ? 16 : 32;
+  s->kb = opts->block > 0 ? opts->block : work < 8000000 ? kSmallBlock : 32;
   // Columns per CTA of the FP64 stencils: 32, halved while the batch gives fewer CTAs than the device has SMs (down to 2:
   // one per thread group).  A W, us at 32 / 16 / 8 / 4 / 2: 7^3 x 32 columns 27.5 / 16.1 / 10.0 / 6.7 / 5.5; 8^3 x 8
   // x 32 28.3 / 16.3 / 10.5 / 9.8 / 14.4; 16^3 x 96 30.8 / 23.1 / 23.2 / 25.7 / 36.6; 24^3 x 160 98 / 104 / 112 / 134 / 201
@@ -371,8 +373,9 @@ int laph_solver_create(laph_solver** out, const laph_problem* probs, int n, cons
       (rc = dalloc(&s->d_ps0, n)) || (rc = dalloc(&s->d_ferr, 1)))
     return fail(rc);
   if (cudaMemset(s->d_ferr, 0, sizeof(int)) != cudaSuccess) return fail(LAPH_ECUDA);
-  // the default filter runs a whole pass as one kernel per extent where the batch is small
-  if (s->fvariant == 1 && s->kb <= 64)
+  // the default filter runs a whole pass as one kernel per extent where the batch is small; a column block or a tile
+  // other than such a batch's own is a request for the step kernels, the only ones that have them
+  if (s->fvariant == 1 && (opts->block == 0 || opts->block == kSmallBlock) && (opts->filter_tile == 0 || opts->filter_tile == 128))
     if (int e = pass_layout(s->hd, opts->link_prec == LAPH_LINKS_BF16, &s->pass)) return fail(e);
   if (!s->pass.empty())
     if (int e = dalloc(&s->d_plan, pass_plan_ints(n))) return fail(e);
