@@ -339,14 +339,17 @@ int laph_autotune_search(const int* deg_c, int nd, const int* block_c, int nb, c
  * probs[0..n): the sample is the first min(n, nsample) problems, links[i] their
  * FP64 host links in `layout`; each setting is timed as the faster of two runs
  * of a solver over the sample (the first also captures its CUDA graphs), a
- * setting that does not converge within opts->max_it is dropped.  model /
+ * setting that does not converge within opts->max_it is dropped.  The sample's
+ * solves run the kernels that the whole batch takes.  model /
  * nmodel: the window model (as laph_solver_set_window_model) when
  * opts->window is LAPH_WINDOW_MLP, else ignored (may be NULL).  Candidates:
  * deg 40, 48, 56, 60, 64, 72, 80, 96 (start: opts->deg, or 60 if <= 1), block 8, 16, 32, 64
- * (start: opts->block, or 32), guard opts->guard, opts->guard + 32 and the fewest
+ * (start: opts->block, or the solver's own), guard opts->guard, opts->guard + 32 and the fewest
  * (>= 4) that give the smallest block width above nev + 4, then the
  * filter's tile of 64, 128 or 256 sites per CTA (start: opts->filter_tile, or
- * 128) with the other three at their best.
+ * 128) with the other three at their best.  A batch whose filter runs whole
+ * passes as one kernel (laph_solve_opts.filter_kernel) has neither block nor
+ * tile: they stay at its 16 and 128.
  * cache_path (may be NULL): a text file of earlier results, one line per
  * device and batch shape; a hit sets opts without timing anything, a new
  * result is appended. */

@@ -15,8 +15,10 @@
 // a candidate kept only when it is more than 1% faster), every setting timed
 // at most once.  laph_solver_autotune times each setting as a real solve of a
 // sample of the batch (the faster of two runs of one solver: the first also
-// captures the CUDA graphs) and keeps the result in an optional cache file,
-// one line per device and batch shape, so a production run tunes once.
+// captures the CUDA graphs), run by the kernels the whole batch takes
+// (batch_form.h), and keeps the result in an optional cache file, one line per
+// device and batch shape, so a production run tunes once.  A batch whose filter
+// runs whole passes as one kernel has no block and no tile to tune.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -29,6 +31,7 @@
 #include <vector>
 
 #include "../../include/laph_gpu.h"
+#include "batch_form.h"
 
 namespace laph {
 void set_error(const char* fmt, ...);
@@ -41,7 +44,7 @@ constexpr double kTuneMargin = 0.01;  // a candidate must be this much faster to
 
 struct SampleCtx {
   const laph_problem* probs;
-  int ns;
+  int n, ns;  // the batch, and how many of it are the sample
   const double* const* links;
   int layout;
   laph_solve_opts base;
@@ -61,7 +64,7 @@ double sample_trial(void* user, int deg, int block, int guard) {
   o.guard = guard;
   o.filter_tile = c->tile;
   laph_solver* s = nullptr;
-  int st = laph_solver_create(&s, c->probs, c->ns, &o, c->device);
+  int st = laph_solver_create_for(&s, c->probs, c->ns, &o, c->device, c->probs, c->n);
   c->last_status = st;
   if (st != LAPH_OK) return -1.0;
   double best = -1.0;
@@ -80,7 +83,10 @@ double sample_trial(void* user, int deg, int block, int guard) {
   return st == LAPH_OK ? best : -1.0;
 }
 
-std::string shape_key(const cudaDeviceProp& prop, const laph_problem* probs, int ns, const laph_solve_opts* o) {
+// The sample's shape and the options, and the batch's form where a solve of the sample by itself would have another
+// (or where passes run as one kernel: block and tile are not tuned then).
+std::string shape_key(const cudaDeviceProp& prop, const laph_problem* probs, int ns, const laph_solve_opts* o,
+                      const laph::BatchForm& sample, const laph::BatchForm& batch) {
   std::string k = prop.name;
   char buf[256];
   std::snprintf(buf, sizeof buf, "|sm_%d%d|", prop.major, prop.minor);
@@ -93,6 +99,13 @@ std::string shape_key(const cudaDeviceProp& prop, const laph_problem* probs, int
                 o->smear_kind, o->smear_p1, o->smear_p2, o->smear_iters, o->smear_compat, o->tol, o->window,
                 o->filter_kernel, o->guard, o->max_it);
   k += buf;
+  if (batch.pass) {
+    k += "|pass";
+  } else if (sample.pass || sample.block != batch.block || sample.cols64 != batch.cols64 ||
+             sample.gram_split != batch.gram_split || sample.kmax != batch.kmax) {
+    std::snprintf(buf, sizeof buf, "|steps%d:%d:%d:%d", batch.block, batch.cols64, batch.gram_split, batch.kmax);
+    k += buf;
+  }
   for (char& ch : k)
     if (ch == '\t' || ch == '\n') ch = ' ';
   return k;
@@ -202,7 +215,15 @@ int laph_solver_autotune(const laph_problem* probs, int n, const double* const* 
     set_error("laph_solver_autotune: cannot query device %d", device);
     return LAPH_ENODEV;
   }
-  const std::string key = shape_key(prop, probs, ns, opts);
+  laph::BatchForm form{}, own{};
+  bool solvable = true;  // else every trial says why it is not
+  for (int i = 0; i < n; ++i) solvable = solvable && probs[i].L >= 3 && probs[i].L <= 128 && probs[i].nev >= 1;
+  if (solvable && opts->guard >= 0) {
+    int e = laph::batch_form(probs, n, opts, device, &form);
+    if (e == LAPH_OK) e = laph::batch_form(probs, ns, opts, device, &own);
+    if (e != LAPH_OK) return e;
+  }
+  const std::string key = shape_key(prop, probs, ns, opts, own, form);
   std::memset(out, 0, sizeof *out);
   if (cache_path && *cache_path && cache_lookup(cache_path, key, out)) {
     out->from_cache = 1;
@@ -213,7 +234,7 @@ int laph_solver_autotune(const laph_problem* probs, int n, const double* const* 
     return LAPH_OK;
   }
   const int deg0 = opts->deg > 1 ? std::min(opts->deg, 96) : 60;
-  const int block0 = opts->block > 0 ? opts->block : 32;
+  const int block0 = form.block > 0 ? form.block : 32;
   const int guard0 = opts->guard;
   const int degs[] = {40, 48, 56, 60, 64, 72, 80, 96};
   const int blocks[] = {8, 16, 32, 64};
@@ -224,8 +245,8 @@ int laph_solver_autotune(const laph_problem* probs, int n, const double* const* 
   if (gmin != guard0 && gmin != guard0 + 32 && ((probs[0].nev + gmin + 31) / 32 != (probs[0].nev + guard0 + 31) / 32))
     guards.push_back(gmin);
   const int tile0 = opts->filter_tile > 0 ? opts->filter_tile : 128;
-  SampleCtx ctx{probs, ns, links, layout, *opts, model, nmodel, device, LAPH_OK, tile0};
-  int st = laph_autotune_search(degs, 8, blocks, 4, guards.data(), (int)guards.size(), deg0, block0, guard0,
+  SampleCtx ctx{probs, n, ns, links, layout, *opts, model, nmodel, device, LAPH_OK, tile0};
+  int st = laph_autotune_search(degs, 8, blocks, form.pass ? 0 : 4, guards.data(), (int)guards.size(), deg0, block0, guard0,
                                 sample_trial, &ctx, out);
   if (st != LAPH_OK) {
     if (ctx.last_status != LAPH_OK && ctx.last_status != LAPH_ENOTCONV)
@@ -236,7 +257,7 @@ int laph_solver_autotune(const laph_problem* probs, int n, const double* const* 
   // the tile axis, with deg / block / guard at their best (the kernel variant
   // with FP32 coefficients per CTA only: wider blocks keep 128 sites)
   out->tile = tile0;
-  if (opts->filter_kernel == 1 && out->block <= 64) {
+  if (opts->filter_kernel == 1 && out->block <= 64 && !form.pass) {
     for (int t : {64, 128, 256}) {
       if (t == tile0) continue;
       ctx.tile = t;

@@ -1,0 +1,24 @@
+// batch_form.h -- the kernels a solver picks by the size of its whole batch.
+// The autotuner times solves of a sample of a batch, which has to run the
+// kernels of the batch, not those a batch as small as the sample would take:
+// it creates its solvers with laph_solver_create_for.
+#pragma once
+#include "../../include/laph_gpu.h"
+
+namespace laph {
+struct BatchForm {
+  int pass;        // the filter runs each whole pass as one kernel per extent
+  int block;       // columns per CTA of the filter's step kernels
+  int cols64;      // columns per CTA of the FP64 block stencils
+  int gram_split;  // the Gram takes its kernel for few units
+  int kmax;        // widest block
+};
+// The form of a batch with these options on `device` (problems and options already checked).
+int batch_form(const laph_problem* batch, int n, const laph_solve_opts* opts, int device, BatchForm* f);
+}  // namespace laph
+
+extern "C" {
+// laph_solver_create for probs[0..n), with the kernels of batch[0..nbatch), of which they are a sample.
+int laph_solver_create_for(laph_solver** out, const laph_problem* probs, int n, const laph_solve_opts* opts, int device,
+                           const laph_problem* batch, int nbatch);
+}

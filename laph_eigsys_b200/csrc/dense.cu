@@ -803,9 +803,10 @@ int dense_init() {
   LAPH_TRY(neglap64_init());
   return small_init();
 }
-int gram(const ProbDesc* pd, const ProbState* ps, const int* start, int np, int nblk, int chunk_rows,
+bool gram_splits(long long units) { return units <= kGramSplitUnits; }
+int gram(const ProbDesc* pd, const ProbState* ps, const int* start, int np, int nblk, int split, int chunk_rows,
          const double2* W, const double2* Y, double2* gpart, cudaStream_t st) {
-  if (nblk <= kGramSplitUnits)
+  if (split)
     k_gram_split<<<4 * nblk, 128, kGramSplitSmem, st>>>(pd, ps, start, np, chunk_rows, W, Y, gpart);
   else
     k_gram<<<nblk, 64, kGramSmem, st>>>(pd, ps, start, np, chunk_rows, W, Y, gpart);

@@ -7,7 +7,9 @@ constexpr int kGramTile = 32;   // block widths k are multiples of this
 constexpr int kRotRows = 128;   // rows per rotation tile
 // Opt the dense kernels into their dynamic shared memory on the current device.
 int dense_init();
-int gram(const ProbDesc* pd, const ProbState* ps, const int* start, int np, int nblk, int chunk_rows,
+// Does a batch of that many (tile pair, row chunk) units take the kernel for few units (split)?
+bool gram_splits(long long units);
+int gram(const ProbDesc* pd, const ProbState* ps, const int* start, int np, int nblk, int split, int chunk_rows,
          const double2* W, const double2* Y, double2* gpart, cudaStream_t st);
 int gram_reduce(const ProbDesc* pd, const ProbState* ps, const int* start, int np, int nblk, const double2* gpart,
                 double2* KK, cudaStream_t st);

@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "batch.cuh"
+#include "batch_form.h"
 #include "common.cuh"
 #include "dense.cuh"
 #include "filter.cuh"
@@ -56,6 +57,7 @@ struct laph_solver {
   int np = 0, mdeg = 16, kb = 32, tile = 128;
   int cols64 = kColsFP64;  // columns per CTA of the FP64 block stencils
   int kmax = 0;                // widest block of the batch
+  int gram_split = 0;          // the Gram's kernel for few units
   int fvariant = 1, lmax = 0;  // filter variant in use (opts.filter_kernel, or 1 where 3 does not apply)
   int* d_ferr = nullptr;       // set by a filter kernel whose bounded wait gave up
   std::vector<PassClass> pass; // layout of the one-kernel filter pass (empty: one kernel per step)
@@ -162,7 +164,66 @@ constexpr int kSmallBlock = 16;  // columns per CTA of the filter for a small ba
 
 int round_up(int a, int b) { return (a + b - 1) / b * b; }
 
+constexpr int kGramChunk = 8192;  // rows of a Gram partial
+
+int check_problems(const laph_problem* probs, int n, const laph_solve_opts* opts) {
+  for (int i = 0; i < n; ++i) {
+    const int L = probs[i].L, nev = probs[i].nev;
+    const int k = round_up(nev + opts->guard, kGramTile);
+    if (L < 3 || L > 128 || nev < 1 || k > 512 || k > 3 * L * L * L / 2) {
+      set_error("laph_solver_create: problem %d: need 3 <= L <= 128, 1 <= nev, block width %d <= min(512, dim/2)", i, k);
+      return LAPH_EINVAL;
+    }
+  }
+  return LAPH_OK;
+}
+
 }  // namespace
+
+namespace laph {
+int batch_form(const laph_problem* batch, int n, const laph_solve_opts* opts, int device, BatchForm* f) {
+  int sms = 0;
+  LAPH_CUDA_TRY(cudaSetDevice(device));
+  LAPH_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+  *f = BatchForm{};
+  std::vector<ProbDesc> d(n);  // what pass_layout reads of a problem
+  long long work = 0, units = 0;
+  for (int i = 0; i < n; ++i) {
+    d[i].L = batch[i].L;
+    d[i].V3 = d[i].L * d[i].L * d[i].L;
+    d[i].k = round_up(batch[i].nev + opts->guard, kGramTile);
+    const int T = d[i].k / kGramTile;
+    work += (long long)d[i].V3 * d[i].k;
+    units += (3LL * d[i].V3 + kGramChunk - 1) / kGramChunk * (T * (T + 1) / 2);
+    f->kmax = std::max(f->kmax, d[i].k);
+  }
+  f->gram_split = gram_splits(units);
+  // Columns per CTA: 32 unless told otherwise, 16 where 32 would leave too few CTAs per step (below 8e6 site-columns;
+  // 24^3 x 2 and 32^3 x 1, 160 columns: 4.1e10 against 3.9e10 site-columns a second, 32^3 x 2: 4.6e10 either way)
+  f->block = opts->block > 0 ? opts->block : work < 8000000 ? kSmallBlock : 32;
+  // Columns per CTA of the FP64 stencils: 32, halved while the batch gives fewer CTAs than the device has SMs (down to 2:
+  // one per thread group).  A W, us at 32 / 16 / 8 / 4 / 2: 7^3 x 32 columns 27.5 / 16.1 / 10.0 / 6.7 / 5.5; 8^3 x 8
+  // x 32 28.3 / 16.3 / 10.5 / 9.8 / 14.4; 16^3 x 96 30.8 / 23.1 / 23.2 / 25.7 / 36.6; 24^3 x 160 98 / 104 / 112 / 134 / 201
+  auto blocks64 = [&](int cols) {
+    long long b = 0;
+    for (const ProbDesc& p : d) b += (long long)((p.V3 + kSites64 - 1) / kSites64) * ((p.k + cols - 1) / cols);
+    return b;
+  };
+  f->cols64 = kColsFP64;
+  while (f->cols64 > 2 && blocks64(f->cols64) < sms) f->cols64 /= 2;
+  // The default filter runs a whole pass as one kernel per extent where the batch is small; a column block or a tile
+  // other than such a batch's own is a request for the step kernels, the only ones that have them.
+  bool variant1 = opts->filter_kernel == 1;
+  if (opts->filter_kernel >= 3)  // what the staged and brick variants cannot take runs as variant 1
+    for (int i = 0; i < n; ++i) variant1 = variant1 || !cheb_staged_ok(d[i].L);
+  if (variant1 && (opts->block == 0 || opts->block == kSmallBlock) && (opts->filter_tile == 0 || opts->filter_tile == 128)) {
+    std::vector<PassClass> pass;
+    LAPH_TRY(pass_layout(d, opts->link_prec == LAPH_LINKS_BF16, &pass));
+    f->pass = !pass.empty();
+  }
+  return LAPH_OK;
+}
+}  // namespace laph
 
 extern "C" {
 
@@ -227,7 +288,12 @@ int laph_solver_destroy(laph_solver* s) {
 }
 
 int laph_solver_create(laph_solver** out, const laph_problem* probs, int n, const laph_solve_opts* opts, int device) {
-  if (!out || !probs || n < 1 || !opts) {
+  return laph_solver_create_for(out, probs, n, opts, device, probs, n);
+}
+
+int laph_solver_create_for(laph_solver** out, const laph_problem* probs, int n, const laph_solve_opts* opts, int device,
+                           const laph_problem* batch, int nbatch) {
+  if (!out || !probs || n < 1 || !opts || !batch || nbatch < n) {
     set_error("laph_solver_create: bad argument");
     return LAPH_EINVAL;
   }
@@ -239,14 +305,8 @@ int laph_solver_create(laph_solver** out, const laph_problem* probs, int n, cons
               "filter_kernel in {0, ..., 5}, filter_tile in {0, 64, 128, 256}, finite direct_resid");
     return LAPH_EINVAL;
   }
-  for (int i = 0; i < n; ++i) {
-    const int L = probs[i].L, nev = probs[i].nev;
-    const int k = round_up(nev + opts->guard, kGramTile);
-    if (L < 3 || L > 128 || nev < 1 || k > 512 || k > 3 * L * L * L / 2) {
-      set_error("laph_solver_create: problem %d: need 3 <= L <= 128, 1 <= nev, block width %d <= min(512, dim/2)", i, k);
-      return LAPH_EINVAL;
-    }
-  }
+  LAPH_TRY(check_problems(probs, n, opts));
+  if (batch != probs) LAPH_TRY(check_problems(batch, nbatch, opts));
   // every argument is checked before the device, so a bad call reports LAPH_EINVAL on any host
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
@@ -263,24 +323,17 @@ int laph_solver_create(laph_solver** out, const laph_problem* probs, int n, cons
   s->o = *opts;
   s->np = n;
   s->mdeg = opts->deg;
-  // Columns per CTA: 32 unless told otherwise, 16 where 32 would leave too few CTAs per step (below 8e6 site-columns;
-  // 24^3 x 2 and 32^3 x 1, 160 columns: 4.1e10 against 3.9e10 site-columns a second, 32^3 x 2: 4.6e10 either way)
-  long long work = 0;
-  for (int i = 0; i < n; ++i) work += (long long)probs[i].L * probs[i].L * probs[i].L * round_up(probs[i].nev + opts->guard, kGramTile);
-  s->kb = opts->block > 0 ? opts->block : work < 8000000 ? kSmallBlock : 32;
-  // Columns per CTA of the FP64 stencils: 32, halved while the batch gives fewer CTAs than the device has SMs (down to 2:
-  // one per thread group).  A W, us at 32 / 16 / 8 / 4 / 2: 7^3 x 32 columns 27.5 / 16.1 / 10.0 / 6.7 / 5.5; 8^3 x 8
-  // x 32 28.3 / 16.3 / 10.5 / 9.8 / 14.4; 16^3 x 96 30.8 / 23.1 / 23.2 / 25.7 / 36.6; 24^3 x 160 98 / 104 / 112 / 134 / 201
-  auto blocks64 = [&](int cols) {
-    long long b = 0;
-    for (int i = 0; i < n; ++i) {
-      const int V3 = probs[i].L * probs[i].L * probs[i].L, k = round_up(probs[i].nev + opts->guard, kGramTile);
-      b += (long long)((V3 + kSites64 - 1) / kSites64) * ((k + cols - 1) / cols);
-    }
-    return b;
-  };
-  s->cols64 = kColsFP64;
-  while (s->cols64 > 2 && blocks64(s->cols64) < 148) s->cols64 /= 2;
+  if (cudaSetDevice(device) != cudaSuccess) {
+    cudaGetLastError();
+    set_error("laph_solver_create: cannot use device %d", device);
+    return fail(LAPH_ECUDA);
+  }
+  BatchForm form;
+  if (int e = batch_form(batch, nbatch, opts, device, &form)) return fail(e);
+  s->kb = form.block;
+  s->cols64 = form.cols64;
+  s->gram_split = form.gram_split;
+  s->kmax = form.kmax;
   // sites per CTA of the filter; the per-thread-coefficient variant and blocks wider than 64 keep 128
   s->tile = opts->filter_tile > 0 && opts->filter_kernel >= 1 && s->kb <= 64 ? opts->filter_tile : 128;
   // the staged variant (3) needs 128-site tiles of whole z-rows inside one plane for every problem
@@ -292,7 +345,7 @@ int laph_solver_create(laph_solver** out, const laph_problem* probs, int n, cons
     if (ok) s->tile = s->fvariant == 4 ? 512 : 128;
     else s->fvariant = 1;
   }
-  if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking) != cudaSuccess) {
+  if (cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking) != cudaSuccess) {
     cudaGetLastError();
     set_error("laph_solver_create: cannot use device %d", device);
     return fail(LAPH_ECUDA);
@@ -320,8 +373,7 @@ int laph_solver_create(laph_solver** out, const laph_problem* probs, int n, cons
     d.gp = o_gp;
     d.rp = o_rp;
     d.tc = o_tc;
-    const int chunk_rows = 8192;
-    d.nchunk = (d.dim + chunk_rows - 1) / chunk_rows;
+    d.nchunk = (d.dim + kGramChunk - 1) / kGramChunk;
     d.nrt = (d.V3 + 127) / 128;  // site tiles of the residual kernel
     const int T = d.k / kGramTile, npair = T * (T + 1) / 2;
     o_u64 += 27LL * d.V3;
@@ -334,7 +386,6 @@ int laph_solver_create(laph_solver** out, const laph_problem* probs, int n, cons
     o_rp += (long long)d.nrt * d.k;
     o_tc += (long long)(s->mdeg + 1) * 3 * d.k;
     s->hd.push_back(d);
-    s->kmax = std::max(s->kmax, d.k);
     max_v3 = std::max(max_v3, (size_t)d.V3);
     const int nst = (d.V3 + 127) / 128;
     per_site.push_back(nst);
@@ -373,9 +424,7 @@ int laph_solver_create(laph_solver** out, const laph_problem* probs, int n, cons
       (rc = dalloc(&s->d_ps0, n)) || (rc = dalloc(&s->d_ferr, 1)))
     return fail(rc);
   if (cudaMemset(s->d_ferr, 0, sizeof(int)) != cudaSuccess) return fail(LAPH_ECUDA);
-  // the default filter runs a whole pass as one kernel per extent where the batch is small; a column block or a tile
-  // other than such a batch's own is a request for the step kernels, the only ones that have them
-  if (s->fvariant == 1 && (opts->block == 0 || opts->block == kSmallBlock) && (opts->filter_tile == 0 || opts->filter_tile == 128))
+  if (form.pass)
     if (int e = pass_layout(s->hd, opts->link_prec == LAPH_LINKS_BF16, &s->pass)) return fail(e);
   if (!s->pass.empty())
     if (int e = dalloc(&s->d_plan, pass_plan_ints(n))) return fail(e);
@@ -485,7 +534,8 @@ static long long rr_launches(const laph_solver* s) { return 7 + small_launches(s
 static int iteration_rr(laph_solver* s, int first_iter) {
   const bool fixed = s->o.window == LAPH_WINDOW_FIXED && s->o.lam_cut > 0.0;
   LAPH_TRY(neglap64_batch(s->d_pd, s->d_ps, s->st_nl, s->np, s->nb_nl, s->cols64, s->U64, s->W, s->Y, s->st));
-  LAPH_TRY(gram(s->d_pd, s->d_ps, s->st_gram, s->np, s->nb_gram, 8192, s->W, s->Y, s->gpart, s->st));
+  LAPH_TRY(gram(s->d_pd, s->d_ps, s->st_gram, s->np, s->nb_gram, s->gram_split, kGramChunk, s->W, s->Y, s->gpart,
+                s->st));
   LAPH_TRY(gram_reduce(s->d_pd, s->d_ps, s->st_gred, s->np, s->nb_gred, s->gpart, s->KK, s->st));
   LAPH_TRY(small_dense(s->d_pd, s->d_ps, s->np, s->kmax, s->KK, s->theta, s->dwork, first_iter, fixed ? 1 : 0,
                        jacobi_sweeps(s), s->tstamp, s->st));
@@ -1310,7 +1360,7 @@ int laph_solver_footprint(const laph_problem* probs, int n, const laph_solve_opt
       set_error("laph_solver_footprint: problem %d is not solvable (see laph_solver_create)", i);
       return LAPH_EINVAL;
     }
-    const long long nchunk = (dim + 8191) / 8192, T = k / kGramTile, npair = T * (T + 1) / 2;
+    const long long nchunk = (dim + kGramChunk - 1) / kGramChunk, T = k / kGramTile, npair = T * (T + 1) / 2;
     const long long mdeg = opts->deg > 0 ? opts->deg : 16;
     o_u64 += 27 * V3;
     o_uf += 27 * V3;
