@@ -43,12 +43,14 @@ __device__ __forceinline__ unsigned long long global_ns() {
 }
 // Wait for phase `parity` of m, giving up after `limit_ns` nanoseconds of the
 // global timer (each try_wait poll suspends the thread for at most a
-// hardware-chosen time); returns false on giving up.
+// hardware-chosen time); returns false on giving up.  The phase is looked at
+// once more after the limit: a thread that was descheduled past it while its
+// copies completed has not failed.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* m, unsigned parity, unsigned long long limit_ns) {
   if (mbar_try_wait(m, parity)) return true;
   const unsigned long long t0 = global_ns();
   while (!mbar_try_wait(m, parity))
-    if (global_ns() - t0 > limit_ns) return false;
+    if (global_ns() - t0 > limit_ns) return mbar_try_wait(m, parity);
   return true;
 }
 // global -> this CTA's shared memory, completing `bytes` on m

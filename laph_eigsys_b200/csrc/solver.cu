@@ -46,6 +46,7 @@ int displace_device(const double2* U, int L, int dir, int nev, long long ldv, co
                     cudaStream_t st);
 int sourceshape_device(const double2* V, int L, int nev, const double* evals, double2* work, double* psi, int cm,
                        cudaStream_t st);
+int sourceshape_copy(const double* dpsi, int L, double* psi, cudaStream_t st);
 }
 
 using namespace laph;
@@ -1289,15 +1290,12 @@ int laph_solver_sourceshape(laph_solver* s, int i, int weighted, double* psi) {
   }
   LAPH_CUDA_TRY(cudaSetDevice(s->dev));
   const ProbDesc& d = s->hd[i];
-  const int H = d.L / 2, Nc = H * H * H;
   // scratch, both free once the run has finished and rewritten by the next run:
-  // W (the class-major copy of the colour-major V), E0 (psi bins)
+  // W (the class-major copy of the colour-major V), E0 (psi bins and a flag)
   double* dpsi = reinterpret_cast<double*>(s->E[0] + d.blk);
   LAPH_TRY(sourceshape_device(s->V + d.blk, d.L, d.nev, weighted ? s->theta + d.kv : nullptr, s->W + d.blk, dpsi, 1,
                               s->st));
-  LAPH_CUDA_TRY(cudaMemcpyAsync(psi, dpsi, sizeof(double) * Nc, cudaMemcpyDeviceToHost, s->st));
-  LAPH_CUDA_TRY(cudaStreamSynchronize(s->st));
-  return LAPH_OK;
+  return sourceshape_copy(dpsi, d.L, psi, s->st);
 }
 
 int laph_solver_displace(laph_solver* s, int i, int dir, double* W, int on_device) {

@@ -35,6 +35,9 @@
 #include "bulk.cuh"
 #include "common.cuh"
 
+// what a source-shape call returns for the kernel's flag (not 0: a bounded wait gave up)
+extern "C" int laph_sourceshape_status(int gave_up);
+
 namespace laph {
 namespace {
 
@@ -123,7 +126,7 @@ constexpr int kSsSmem =
 constexpr unsigned long long kSsWaitNs = 1000000000ull;  // 1 s: a stage that takes longer is a fault
 
 __global__ void __launch_bounds__(512, 1) k_ss_tile(const double2* __restrict__ Vp, int L, int nev,
-                                                    double* __restrict__ psi) {
+                                                    double* __restrict__ psi, int* gave_up) {
   const int H = L / 2, Nc = H * H * H, R = 3 * Nc;
   const int T = (Nc + kSsSites - 1) / kSsSites;
   const int ntile = 8 * (T * (T + 1) / 2), nstep = (nev + kSsK - 1) / kSsK;
@@ -179,9 +182,9 @@ __global__ void __launch_bounds__(512, 1) k_ss_tile(const double2* __restrict__ 
       for (int j = 0; j < 3; ++j) accr[i][j][0] = accr[i][j][1] = acci[i][j][0] = acci[i][j][1] = 0.0;
     for (int it = 0; it < nstep; ++it) {
       const bool ok = mbar_wait_bounded(&mbar[st], par, kSsWaitNs);
-      if (__syncthreads_or(!ok)) {  // gave up: no value of psi stands, and no copy may outlive the CTA
+      if (__syncthreads_or(!ok)) {  // gave up: psi is not valid, and no copy may outlive the CTA
         for (int s = 0; s < kSsStages; ++s) mbar_wait_bounded(&mbar[s], s < st ? par ^ 1u : par, kSsWaitNs);
-        for (int b = threadIdx.x; b < Nc; b += blockDim.x) psi[b] = __longlong_as_double(-1LL);
+        if (threadIdx.x == 0) *gave_up = 1;
         return;
       }
       // every warp is past the stage that is refilled now
@@ -375,8 +378,9 @@ bool ss_use_dmma() {
 
 }  // namespace
 
-// psi[(L/2)^3] (device) from a device eigensystem V [3 V3][nev] (column stride 3 V3,
-// colour-major rows when cm); work: 8 nev (3 V3 / 8) double2 of device scratch owned by the caller.
+// psi[(L/2)^3 + 1] (device) from a device eigensystem V [3 V3][nev] (column stride 3 V3,
+// colour-major rows when cm); work: 8 nev (3 V3 / 8) double2 of device scratch owned by the caller.  The element past
+// the bins holds an int, not 0 where a bounded wait of the kernel gave up: sourceshape_copy reads both back.
 int sourceshape_device(const double2* V, int L, int nev, const double* evals, double2* work, double* psi, int cm,
                        cudaStream_t st) {
   int dev = 0;
@@ -390,22 +394,41 @@ int sourceshape_device(const double2* V, int L, int nev, const double* evals, do
   }
   const int H = L / 2, Nc = H * H * H;
   const int T = (Nc + kSsSites - 1) / kSsSites;
-  LAPH_CUDA_TRY(cudaMemsetAsync(psi, 0, sizeof(double) * Nc, st));
+  LAPH_CUDA_TRY(cudaMemsetAsync(psi, 0, sizeof(double) * (Nc + 1), st));
   const long long total = 8LL * nev * 3 * Nc;
   const int pb = (int)std::min<long long>((total + 255) / 256, 148LL * 16);
   k_ss_pack<<<pb, 256, 0, st>>>(V, L, nev, evals, work, cm);
   LAPH_CUDA_TRY(cudaGetLastError());
   if (ss_use_dmma())
-    k_ss_tile<<<std::min(8 * T * (T + 1) / 2, sms), 512, kSsSmem, st>>>(work, L, nev, psi);
+    k_ss_tile<<<std::min(8 * T * (T + 1) / 2, sms), 512, kSsSmem, st>>>(work, L, nev, psi,
+                                                                            reinterpret_cast<int*>(psi + Nc));
   else
     k_ss_tile_fma<<<8 * T * (T + 1) / 2, 512, kSsFmaSmem, st>>>(work, L, nev, psi);
   LAPH_CUDA_TRY(cudaGetLastError());
   return LAPH_OK;
 }
 
+// The bins of sourceshape_device to the host, once its work on st is done.
+int sourceshape_copy(const double* dpsi, int L, double* psi, cudaStream_t st) {
+  const int H = L / 2, Nc = H * H * H;
+  std::vector<double> h(Nc + 1);  // bins and flag in one copy
+  LAPH_CUDA_TRY(cudaMemcpyAsync(h.data(), dpsi, sizeof(double) * (Nc + 1), cudaMemcpyDeviceToHost, st));
+  LAPH_CUDA_TRY(cudaStreamSynchronize(st));
+  int gave_up;
+  std::memcpy(&gave_up, &h[Nc], sizeof gave_up);
+  std::memcpy(psi, h.data(), sizeof(double) * Nc);
+  return laph_sourceshape_status(gave_up);
+}
+
 }  // namespace laph
 
 using namespace laph;
+
+extern "C" int laph_sourceshape_status(int gave_up) {
+  if (!gave_up) return LAPH_OK;
+  set_error("laph_sourceshape: a bounded wait of the tile kernel gave up; psi is not valid");
+  return LAPH_ECUDA;
+}
 
 extern "C" int laph_sourceshape(const double* V, int L, int nev, const double* evals, int on_device, double* psi,
                                 int device) {
@@ -438,7 +461,7 @@ extern "C" int laph_sourceshape(const double* V, int L, int nev, const double* e
   };
   if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess ||
       cudaMalloc(&work, sizeof(double2) * dim * nev) != cudaSuccess ||
-      cudaMalloc(&dpsi, sizeof(double) * Nc) != cudaSuccess) {
+      cudaMalloc(&dpsi, sizeof(double) * (Nc + 1)) != cudaSuccess) {
     cudaGetLastError();
     cleanup();
     set_error("laph_sourceshape: device allocation failed");
@@ -465,11 +488,7 @@ extern "C" int laph_sourceshape(const double* V, int L, int nev, const double* e
     ev_use = dev_ev;
   }
   rc = sourceshape_device(Vuse, L, nev, ev_use, work, dpsi, 0, st);
-  if (rc == LAPH_OK && (cudaMemcpyAsync(psi, dpsi, sizeof(double) * Nc, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-                        cudaStreamSynchronize(st) != cudaSuccess)) {
-    set_error("laph_sourceshape: %s", cudaGetErrorString(cudaGetLastError()));
-    rc = LAPH_ECUDA;
-  }
+  if (rc == LAPH_OK) rc = sourceshape_copy(dpsi, L, psi, st);
   cleanup();
   return rc;
 }
