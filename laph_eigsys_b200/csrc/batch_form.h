@@ -1,7 +1,8 @@
 // batch_form.h -- the kernels a solver picks by the size of its whole batch.
 // The autotuner times solves of a sample of a batch, which has to run the
 // kernels of the batch, not those a batch as small as the sample would take:
-// it creates its solvers with laph_solver_create_for.
+// it creates its solvers with laph_solver_create_for.  Exported, but not part of
+// the public interface.
 #pragma once
 #include "../../include/laph_gpu.h"
 
@@ -21,4 +22,7 @@ extern "C" {
 // laph_solver_create for probs[0..n), with the kernels of batch[0..nbatch), of which they are a sample.
 int laph_solver_create_for(laph_solver** out, const laph_problem* probs, int n, const laph_solve_opts* opts, int device,
                            const laph_problem* batch, int nbatch);
+// Blocks wider than `width` run their Jacobi in global memory, as they do on a device without room for their clusters
+// (for the tests; before the solver's first run).
+int laph_solver_limit_jacobi(laph_solver* s, int width);
 }

@@ -15,14 +15,16 @@ int gram_reduce(const ProbDesc* pd, const ProbState* ps, const int* start, int n
                 double2* KK, cudaStream_t st);
 // Per problem, from G and H: projection against the frozen columns, Cholesky, inverse, projected matrix, Jacobi
 // (at most max_sweeps sweeps), sort, the rotation's coefficients C (fifth k x k matrix of KK), next window
-// (small.cu); kmax: the batch's widest block.  tstamp[p][0..kSmallPhases-1] receives the global timer (ns) at the
+// (small.cu); kmax: the batch's widest block, smem_n: the widest whose Jacobi runs in shared memory.  tstamp[p][0..kSmallPhases-1] receives the global timer (ns) at the
 // phase boundaries.
 constexpr int kSmallPhases = 7;
 int small_init();
-int small_dense(const ProbDesc* pd, ProbState* ps, int np, int kmax, double2* KK, double* theta, double* dwork,
+// The widest block whose Jacobi this device can run in the shared memory of a thread-block cluster (0: none).
+int small_jacobi_width(int* n);
+int small_dense(const ProbDesc* pd, ProbState* ps, int np, int kmax, int smem_n, double2* KK, double* theta, double* dwork,
                 int first_iter, int fixed_cut, int max_sweeps, unsigned long long* tstamp, cudaStream_t st);
 // kernels one small_dense call launches
-int small_launches(int kmax, int max_sweeps);
+int small_launches(int kmax, int smem_n, int max_sweeps);
 // Chebyshev coefficient table and S scaling for a filter of degree m (or *dm
 // when dm is not null: the degree the device-side loop chose).
 int coef(const ProbDesc* pd, const ProbState* ps, int np, const double* theta, double* tcoef, double* scol, int m,

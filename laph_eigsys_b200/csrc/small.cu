@@ -494,8 +494,9 @@ __global__ void __launch_bounds__(256) k_prod(const ProbDesc* __restrict__ pd, c
 // computes all n/2 rotations of a step itself, from the owners' diagonal entries
 // (three distributed shared memory reads per pair), so a step has one cluster
 // barrier and one CTA barrier.  The product of the rotations is not kept here:
-// they go to a log that k_apply replays.  n > kJacSmemN keeps both
-// copies in global memory (Ht and the Cholesky factor's storage), same code.
+// they go to a log that k_apply replays.  n > kJacSmemN16, or a cluster the
+// device has no room for, keeps both copies in global memory (Ht and the
+// Cholesky factor's storage), same code.
 // A step costs 1.4-3.9 us (n = 64 .. 320) where one SM took 4.3-50 us; much of it is
 // the chain of square roots and divisions of a rotation.  The test for a rotation needs
 // no square root of its own, and up to n = 128 and in global memory (SPLIT) one half
@@ -902,12 +903,39 @@ int small_init() {
   return LAPH_OK;
 }
 
-int small_launches(int kmax, int max_sweeps) {
-  const int per = kmax > kJacSmemN16 ? 1 : 2;
+// A cluster of 16 CTAs of up to 215 KB, or of 8 of up to 210 KB, may have no room on the device (fewer SMs in every GPC,
+// as in a partitioned one); its blocks then take the global-memory form.
+int small_jacobi_width(int* n) {
+  auto fits = [](const void* fn, int c, int smem) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(c);
+    cfg.blockDim = dim3(kJacThreads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = c;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    return clusters > 0;
+  };
+  *n = !fits((const void*)k_jacobi<8, true, false>, 8, 4 * kJacSmemN8 * kJacSmemN8)       ? 0
+       : !fits((const void*)k_jacobi<16, true, false>, 16, 2 * kJacSmemN16 * kJacSmemN16) ? kJacSmemN8
+                                                                                          : kJacSmemN16;
+  return LAPH_OK;
+}
+
+int small_launches(int kmax, int smem_n, int max_sweeps) {
+  const int per = kmax > smem_n ? 1 : 2;
   return 7 + 2 * ((max_sweeps + per - 1) / per);
 }
 
-int small_dense(const ProbDesc* pd, ProbState* ps, int np, int kmax, double2* KK, double* theta, double* dwork,
+int small_dense(const ProbDesc* pd, ProbState* ps, int np, int kmax, int smem_n, double2* KK, double* theta, double* dwork,
                 int first_iter, int fixed_cut, int max_sweeps, unsigned long long* tstamp, cudaStream_t st) {
   const int T = kmax / NB;
   const dim3 tiles(T * T, np);
@@ -922,20 +950,20 @@ int small_dense(const ProbDesc* pd, ProbState* ps, int np, int kmax, double2* KK
   LAPH_CUDA_TRY(cudaGetLastError());
   // The log holds two sweeps, or one where the Jacobi's second copy takes the Cholesky factor's storage and Q
   // the second sweep's log: more sweeps run as further launches on the rotated matrix.
-  const int global = kmax > kJacSmemN16, per = global ? 1 : 2;
+  const int global = kmax > smem_n, per = global ? 1 : 2;
   for (int s = 0; s < max_sweeps; s += per) {
     const int ns = std::min(per, max_sweeps - s), last = s + per >= max_sweeps;
-    if (kmax <= kJacSplitN)
+    if (global)
+      LAPH_TRY((launch_jacobi<8, false, true>(pd, ps, np, 0, KK, theta, dwork, first_iter, fixed_cut, ns, last, tstamp, st)));
+    else if (kmax <= kJacSplitN)
       LAPH_TRY((launch_jacobi<8, true, true>(pd, ps, np, 4 * kmax * kmax, KK, theta, dwork, first_iter, fixed_cut, ns,
                                              last, tstamp, st)));
     else if (kmax <= kJacSmemN8)
       LAPH_TRY((launch_jacobi<8, true, false>(pd, ps, np, 4 * kmax * kmax, KK, theta, dwork, first_iter, fixed_cut, ns, last,
                                        tstamp, st)));
-    else if (!global)
+    else
       LAPH_TRY((launch_jacobi<16, true, false>(pd, ps, np, 2 * kmax * kmax, KK, theta, dwork, first_iter, fixed_cut, ns, last,
                                         tstamp, st)));
-    else
-      LAPH_TRY((launch_jacobi<8, false, true>(pd, ps, np, 0, KK, theta, dwork, first_iter, fixed_cut, ns, last, tstamp, st)));
     const dim3 rows((kmax + kApplyRows - 1) / kApplyRows, np);
     auto apply = kmax <= 160 ? k_apply<5> : kmax <= 256 ? k_apply<8> : k_apply<16>;
     apply<<<rows, kApplyThreads, apply_smem(kmax), st>>>(pd, ps, KK, theta, dwork, s == 0, last, global, tstamp);

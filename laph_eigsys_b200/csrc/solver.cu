@@ -58,6 +58,7 @@ struct laph_solver {
   int np = 0, mdeg = 16, kb = 32, tile = 128;
   int cols64 = kColsFP64;  // columns per CTA of the FP64 block stencils
   int kmax = 0;                // widest block of the batch
+  int jacobi_n = 0;            // widest block whose Jacobi runs in shared memory
   int gram_split = 0;          // the Gram's kernel for few units
   int fvariant = 1, lmax = 0;  // filter variant in use (opts.filter_kernel, or 1 where 3 does not apply)
   int* d_ferr = nullptr;       // set by a filter kernel whose bounded wait gave up
@@ -352,6 +353,7 @@ int laph_solver_create_for(laph_solver** out, const laph_problem* probs, int n, 
     return fail(LAPH_ECUDA);
   }
   if (int e = dense_init()) return fail(e);
+  if (int e = small_jacobi_width(&s->jacobi_n)) return fail(e);
   if (int e = cheb_init()) return fail(e);
   // descriptors and pool offsets
   long long o_u64 = 0, o_uf = 0, o_sc = 0, o_blk = 0, o_kk = 0, o_kv = 0, o_gp = 0, o_rp = 0, o_tc = 0;
@@ -530,7 +532,7 @@ static int residual(laph_solver* s) {
 
 static int jacobi_sweeps(const laph_solver* s) { return s->o.jacobi_sweeps > 0 ? s->o.jacobi_sweeps : 2; }
 // kernels of one iteration_rr: A W, Gram, its reduction, the small step, rotation, residual, zero, check
-static long long rr_launches(const laph_solver* s) { return 7 + small_launches(s->kmax, jacobi_sweeps(s)); }
+static long long rr_launches(const laph_solver* s) { return 7 + small_launches(s->kmax, s->jacobi_n, jacobi_sweeps(s)); }
 
 static int iteration_rr(laph_solver* s, int first_iter) {
   const bool fixed = s->o.window == LAPH_WINDOW_FIXED && s->o.lam_cut > 0.0;
@@ -538,7 +540,7 @@ static int iteration_rr(laph_solver* s, int first_iter) {
   LAPH_TRY(gram(s->d_pd, s->d_ps, s->st_gram, s->np, s->nb_gram, s->gram_split, kGramChunk, s->W, s->Y, s->gpart,
                 s->st));
   LAPH_TRY(gram_reduce(s->d_pd, s->d_ps, s->st_gred, s->np, s->nb_gred, s->gpart, s->KK, s->st));
-  LAPH_TRY(small_dense(s->d_pd, s->d_ps, s->np, s->kmax, s->KK, s->theta, s->dwork, first_iter, fixed ? 1 : 0,
+  LAPH_TRY(small_dense(s->d_pd, s->d_ps, s->np, s->kmax, s->jacobi_n, s->KK, s->theta, s->dwork, first_iter, fixed ? 1 : 0,
                        jacobi_sweeps(s), s->tstamp, s->st));
   LAPH_TRY(rotate(s->d_pd, s->d_ps, s->st_rot, s->np, s->nb_rot, s->W, s->KK, s->V, s->st));
   LAPH_TRY(residual(s));
@@ -1264,6 +1266,16 @@ int laph_solver_stream(laph_solver* s, void** stream) {
 int laph_solver_timings(laph_solver* s, double* ms4) {
   if (!s || !ms4) return LAPH_EINVAL;
   for (int i = 0; i < 4; ++i) ms4[i] = s->ms[i];
+  return LAPH_OK;
+}
+
+int laph_solver_limit_jacobi(laph_solver* s, int width) {
+  if (!s || s->ran || width < 0) {
+    set_error("laph_solver_limit_jacobi: bad argument or solver has run");
+    return LAPH_EINVAL;
+  }
+  // as on a device with no room for the clusters of wider blocks
+  if (width < s->jacobi_n) s->jacobi_n = width;
   return LAPH_OK;
 }
 
