@@ -791,7 +791,9 @@ __device__ __forceinline__ void apply_rows(const Small& v, double2* Q, int row, 
     __syncthreads();
   }
   cp_async_wait<0>();
-  // the row is in registers, so it can go back in place: Ritz order at the end, else position order
+  // The row is in registers, so it can go back in place: Ritz order at the end, else position order.  A launch without a
+  // step comes here with nothing else between the lanes' reads and their permuted writes.
+  __syncwarp();
 #pragma unroll
   for (int i = 0; i < M; ++i) {
     const int p = lane * M + i, q = n - 1 - p;

@@ -23,9 +23,11 @@ def _solve(gpu, probs, limit=None, sweeps=2, tol=1e-10):
     return out
 
 
-# widths 32, 128, 224 (clusters of 8), 256 and 320 (of 16)
+# widths 32, 128, 224 (clusters of 8), 256 and 320 (of 16); at six sweeps the last launches find the matrix diagonal and
+# only bring the rows into Ritz order, in place
 @pytest.mark.parametrize("nev,limit,sweeps", [(12, 0, 2), (112, 0, 2), (112, 0, 3), (208, 0, 2), (240, 224, 2), (240, 0, 3),
-                                              (304, 224, 2)])
+                                              (304, 224, 2),
+                                              (40, 0, 6), (208, 0, 6)])
 def test_without_room_for_clusters_the_bits_are_the_same(gpu, nev, limit, sweeps):
     a, b = (_solve(gpu, [(8, nev)], limit=l, sweeps=sweeps) for l in (None, limit))
     assert all(np.array_equal(x, y) for x, y in zip(a[0], b[0]))
