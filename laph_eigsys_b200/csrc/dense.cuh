@@ -24,7 +24,7 @@ int small_jacobi_width(int* n);
 int small_dense(const ProbDesc* pd, ProbState* ps, int np, int kmax, int smem_n, double2* KK, double* theta, double* dwork,
                 int first_iter, int fixed_cut, int max_sweeps, unsigned long long* tstamp, cudaStream_t st);
 // kernels one small_dense call launches
-int small_launches(int kmax, int smem_n, int max_sweeps);
+int small_launches(int np, int kmax, int smem_n, int max_sweeps);
 // Chebyshev coefficient table and S scaling for a filter of degree m (or *dm
 // when dm is not null: the degree the device-side loop chose).
 int coef(const ProbDesc* pd, const ProbState* ps, int np, const double* theta, double* tcoef, double* scol, int m,

@@ -1,4 +1,5 @@
 // links.cu -- boundary link layouts and plaquette reductions.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 
@@ -176,7 +177,10 @@ __global__ void k_plaq_finish(const double* __restrict__ mom, int nts, double in
 
 int plaquette_moments_batch(const double2* U, int L, int nts, double* vals, double* out, cudaStream_t st) {
   const Lat g = make_lat(L);
-  k_plaq_vals<<<dim3(ceil_div(g.V3, 128), 3, nts), 128, 0, st>>>(U, g, (size_t)27 * g.V3, vals);
+  constexpr int kMaxGridZ = 65535;
+  for (int t = 0; t < nts; t += kMaxGridZ)
+    k_plaq_vals<<<dim3(ceil_div(g.V3, 128), 3, std::min(kMaxGridZ, nts - t)), 128, 0, st>>>(
+        U + (size_t)t * 27 * g.V3, g, (size_t)27 * g.V3, vals + (size_t)t * 3 * g.V3);
   k_plaq_moments<<<nts, 512, 0, st>>>(vals, g.V3, out);
   LAPH_CUDA_TRY(cudaGetLastError());
   return LAPH_OK;

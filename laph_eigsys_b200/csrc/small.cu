@@ -932,13 +932,21 @@ int small_jacobi_width(int* n) {
   return LAPH_OK;
 }
 
-int small_launches(int kmax, int smem_n, int max_sweeps) {
-  const int per = kmax > smem_n ? 1 : 2;
-  return 7 + 2 * ((max_sweeps + per - 1) / per);
+// Problems of one launch: they are grid rows, of which there are 65535 at most.
+constexpr int kSmallMaxProbs = 65535;
+
+int small_launches(int np, int kmax, int smem_n, int max_sweeps) {
+  const int per = kmax > smem_n ? 1 : 2, groups = (np + kSmallMaxProbs - 1) / kSmallMaxProbs;
+  return groups * (7 + 2 * ((max_sweeps + per - 1) / per));
 }
 
 int small_dense(const ProbDesc* pd, ProbState* ps, int np, int kmax, int smem_n, double2* KK, double* theta, double* dwork,
                 int first_iter, int fixed_cut, int max_sweeps, unsigned long long* tstamp, cudaStream_t st) {
+  if (np > kSmallMaxProbs) {
+    LAPH_TRY(small_dense(pd + kSmallMaxProbs, ps + kSmallMaxProbs, np - kSmallMaxProbs, kmax, smem_n, KK, theta, dwork,
+                         first_iter, fixed_cut, max_sweeps, tstamp + (size_t)kSmallMaxProbs * kSmallPhases, st));
+    np = kSmallMaxProbs;
+  }
   const int T = kmax / NB;
   const dim3 tiles(T * T, np);
   k_project<<<tiles, 256, kProjSmem, st>>>(pd, ps, KK, theta, dwork);

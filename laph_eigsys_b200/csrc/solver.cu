@@ -532,7 +532,7 @@ static int residual(laph_solver* s) {
 
 static int jacobi_sweeps(const laph_solver* s) { return s->o.jacobi_sweeps > 0 ? s->o.jacobi_sweeps : 2; }
 // kernels of one iteration_rr: A W, Gram, its reduction, the small step, rotation, residual, zero, check
-static long long rr_launches(const laph_solver* s) { return 7 + small_launches(s->kmax, s->jacobi_n, jacobi_sweeps(s)); }
+static long long rr_launches(const laph_solver* s) { return 7 + small_launches(s->np, s->kmax, s->jacobi_n, jacobi_sweeps(s)); }
 
 static int iteration_rr(laph_solver* s, int first_iter) {
   const bool fixed = s->o.window == LAPH_WINDOW_FIXED && s->o.lam_cut > 0.0;
