@@ -295,9 +295,12 @@ int laph_solver_counters(laph_solver* s, long long* c3);
 /* Algorithmic bytes of the last run's filter passes (lap_cheb_mrhs): b2[0] =
  * what the correction-form recurrence must move (per unlocked site-vector and
  * step 24 B for each of X, Z, S read and Y written, the last step FP64 V read
- * and W written, W = V for locked columns, the links once per column block),
+ * and W written, W = V for locked columns, the links once per column block and
+ * step, or once per problem and pass where a pass is one kernel),
  * b2[1] = the plain recurrence's unit, 72 B per site-vector-step (X, Z read, Y
- * written) plus the links once per column block. */
+ * written) plus the same links.  Where a pass is one kernel the vectors stay in
+ * L2 between its steps: the bytes say what its loads and stores move, not HBM
+ * traffic. */
 int laph_solver_filter_bytes(laph_solver* s, double* b2);
 /* How the last run looped: device_loop = 1 when the whole solve was one
  * graph launch (the WHILE node on the device), 0 when the host drove the

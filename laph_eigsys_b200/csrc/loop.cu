@@ -99,15 +99,16 @@ __global__ void k_loop_pass_begin(const ProbDesc* __restrict__ pd, ProbState* __
     if (!S.active) continue;
     const ProbDesc d = pd[p];
     const int nl = S.nlock, nact = d.k - nl;
-    const int nblk = (d.k + lp.kb - 1) / lp.kb - nl / lp.kb;
+    // reads of a problem's links: once a pass, or per step and column block
+    const double lreads = lp.pass ? 1.0 : (double)((d.k + lp.kb - 1) / lp.kb - nl / lp.kb) * (m - 1);
     double per = S.direct ? 72.0 : 0.0;  // a direct pass starts with S = FP32(V)
     for (int n = 1; n < m; ++n) {
       const int reads = n == 1 ? 1 : (n == 2 ? 2 : (nos ? 2 : 3));
       per += reads * 24.0 + (n == m - 1 ? 96.0 : 24.0);
     }
     atomicAdd(&s_sv, (double)d.V3 * nact * (m - 1));
-    atomicAdd(&s_b0, (double)d.V3 * (nact * per + nl * 96.0 + (double)nblk * (m - 1) * lp.lbytes));
-    atomicAdd(&s_b1, (double)d.V3 * (m - 1) * (nact * 72.0 + (double)nblk * lp.lbytes));
+    atomicAdd(&s_b0, (double)d.V3 * (nact * per + nl * 96.0 + lreads * lp.lbytes));
+    atomicAdd(&s_b1, (double)d.V3 * ((m - 1) * (nact * 72.0) + lreads * lp.lbytes));
   }
   // the filter steps of this pass: n = 1..m-2 middle (0), n = m-1 the last (1), the same without S (2, 3) for
   // n >= 3 of an all-direct pass, none beyond (4: past the last branch of every SWITCH)

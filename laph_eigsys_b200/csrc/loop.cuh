@@ -28,8 +28,9 @@ struct LoopParams {
   int mdeg;          // degree cap of every pass
   int max_it;        // passes run while it < max_it
   int kb;            // filter columns per CTA
+  int pass;          // a pass is one kernel, which reads a problem's links once
   int mlp;           // window = learned: check its first pass
-  double lbytes;     // filter link bytes per site per column block
+  double lbytes;     // filter link bytes per site
   double lam_top;    // exact upper bound of the spectrum (12 or opts.lam_max)
   double cap_resid;  // degree cap while the largest wanted residual exceeds this
   double win_check;  // the learned window's check after its first pass

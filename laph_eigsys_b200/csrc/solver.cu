@@ -95,8 +95,9 @@ struct laph_solver {
   long long cnt[3] = {0, 0, 0};
   // algorithmic bytes of the filter passes of the last run: [0] what the
   // kernels must move (X, Z, S read, Y written, FP64 V / W in the last step,
-  // W = V for locked columns, links once per column block), [1] the unit
-  // 72 B + links / block per unlocked site-vector-step (X, Z read, Y written)
+  // W = V for locked columns, links once per column block and step, or once per
+  // problem where a pass is one kernel), [1] the unit 72 B per unlocked
+  // site-vector-step (X, Z read, Y written) and the same links
   double fbytes[2] = {0, 0};
   std::vector<cudaEvent_t> evf;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
@@ -804,6 +805,7 @@ static int build_solve_graph(laph_solver* s) {
   lp.mdeg = s->mdeg;
   lp.max_it = o.max_it;
   lp.kb = s->kb;
+  lp.pass = !s->pass.empty();
   lp.mlp = o.window == LAPH_WINDOW_MLP;
   lp.lbytes = o.link_prec == LAPH_LINKS_BF16 ? 112.0 : 216.0;
   lp.lam_top = o.lam_max > 0.0 ? o.lam_max : 12.0;
@@ -1058,20 +1060,21 @@ int laph_solver_run(laph_solver* s, laph_result* res) {
     }
     const bool nos = nact_p > 0 && ndir_p == nact_p;
     LAPH_CUDA_TRY(cudaMemcpyAsync(s->d_ps, s->hps.data(), s->np * sizeof(ProbState), cudaMemcpyHostToDevice, s->st));
-    const double lbytes = s->o.link_prec == LAPH_LINKS_BF16 ? 112.0 : 216.0;  // per site per column block
+    const double lbytes = s->o.link_prec == LAPH_LINKS_BF16 ? 112.0 : 216.0;  // per site
     for (int i = 0; i < s->np; ++i) {
       if (!s->hps[i].active) continue;
       const ProbDesc& d = s->hd[i];
       const int nl = s->hps[i].nlock, nact = d.k - nl;
       s->cnt[0] += (long long)d.V3 * nact * (m - 1);
-      const int nblk = (d.k + s->kb - 1) / s->kb - nl / s->kb;  // column blocks with an unlocked column
+      // reads of the links: once a pass, or per step and column block with an unlocked column
+      const double lreads = s->pass.empty() ? (double)((d.k + s->kb - 1) / s->kb - nl / s->kb) * (m - 1) : 1.0;
       double per = s->hps[i].direct ? 72.0 : 0.0;  // bytes per unlocked site-vector over the pass
       for (int n = 1; n < m; ++n) {
         const int reads = n == 1 ? 1 : (n == 2 ? 2 : (nos ? 2 : 3));
         per += reads * 24.0 + (n == m - 1 ? 96.0 : 24.0);
       }
-      s->fbytes[0] += (double)d.V3 * (nact * per + nl * 96.0 + (double)nblk * (m - 1) * lbytes);
-      s->fbytes[1] += (double)d.V3 * (m - 1) * (nact * 72.0 + (double)nblk * lbytes);
+      s->fbytes[0] += (double)d.V3 * (nact * per + nl * 96.0 + lreads * lbytes);
+      s->fbytes[1] += (double)d.V3 * ((m - 1) * (nact * 72.0) + lreads * lbytes);
     }
     s->cnt[1] += filter_launches(s, m);
     s->degs.push_back(m);

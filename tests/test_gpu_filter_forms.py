@@ -94,3 +94,23 @@ def test_step_kernels_under_the_checked_build(gpu, tmp_path):
             assert np.abs(got[f"ev{tile}_{i}"] - ev).max() <= 1e-10 * 12.0
             overlap = np.abs(got[f"v{tile}_{i}"].conj().T @ V)
             assert np.abs(np.linalg.norm(overlap, axis=0) - 1.0).max() <= 1e-6
+
+
+@pytest.mark.parametrize("loop", [0, 1], ids=["device loop", "host loop"])
+@pytest.mark.parametrize("prec,lbytes", [("fp32", 216), ("bf16", 112)])
+def test_filter_bytes_count_the_links_the_form_reads(gpu, prec, lbytes, loop):
+    """One filter pass (after the first Rayleigh-Ritz) over 32 unlocked columns of 8^3: the same steps in both forms,
+    whose links are read once, or per step and block of 16 columns."""
+    got = {}
+    for name, kw in (("pass", {}), ("steps", {"block": 16, "filter_tile": 64})):
+        s = gpu.Solver([(8, 20)], guard=12, tol=1e-10, deg=12, max_it=2, host_loop=loop,
+                       link_prec=gpu.LINKS_BF16 if prec == "bf16" else gpu.LINKS_FP32, **kw)
+        s.set_links(0, random_links(8, 0.4, 5700))
+        s.run()
+        got[name] = s.counters()[0], s.filter_bytes()
+        s.close()
+    assert got["pass"][0] == got["steps"][0] and got["pass"][0] % (8 ** 3 * 32) == 0
+    steps = got["pass"][0] // (8 ** 3 * 32)
+    assert steps >= 1
+    for a, b in zip(got["steps"][1], got["pass"][1]):
+        assert a - b == 8 ** 3 * lbytes * (2 * steps - 1)
