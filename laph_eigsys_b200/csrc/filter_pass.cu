@@ -331,11 +331,21 @@ __global__ void __launch_bounds__(kPassThreads, 2)
 
 size_t pass_plan_ints(int np) { return plan_ctr(np) + (size_t)kPassClasses * kMaxTeams * kPassLine; }
 
+bool pass_small(const std::vector<ProbDesc>& probs) {
+  long long work = 0;
+  int extents = 0, seen[kPassClasses] = {};
+  for (const ProbDesc& d : probs) {
+    work += (long long)d.V3 * d.k;
+    if (std::find(seen, seen + extents, d.L) != seen + extents) continue;
+    if (extents == kPassClasses) return false;
+    seen[extents++] = d.L;
+  }
+  return work <= kPassMaxWork;
+}
+
 int pass_layout(const std::vector<ProbDesc>& probs, int bf16, std::vector<PassClass>* out) {
   out->clear();
-  long long work = 0;
-  for (const ProbDesc& d : probs) work += (long long)d.V3 * d.k;
-  if (work > kPassMaxWork) return LAPH_OK;
+  if (!pass_small(probs)) return LAPH_OK;
   int dev = 0, sms = 0, occ = 0;
   const void* fn = bf16 ? (const void*)k_cheb_pass<__nv_bfloat162> : (const void*)k_cheb_pass<float2>;
   LAPH_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kPassSmem));
@@ -348,7 +358,6 @@ int pass_layout(const std::vector<ProbDesc>& probs, int bf16, std::vector<PassCl
     size_t c = 0;
     while (c < cls.size() && cls[c].L != d.L) ++c;
     if (c == cls.size()) {
-      if (c == (size_t)kPassClasses) return LAPH_OK;
       // sites per CTA: the tile whose teams keep the most sites in flight per step time (a step takes as long as a
       // tile has sites, plus about 16 sites' worth of waiting)
       PassClass g{d.L, 0, 0, 0, 0};

@@ -19,6 +19,7 @@ struct PassClass {
 // ones (an extent whose sites outnumber the co-resident threads, or more than
 // kPassClasses extents).
 constexpr int kPassClasses = 4;
+bool pass_small(const std::vector<ProbDesc>& probs);  // few enough site-columns and extents for it (reads L, V3 and k)
 int pass_layout(const std::vector<ProbDesc>& probs, int bf16, std::vector<PassClass>* out);
 // ints of plan scratch for np problems
 size_t pass_plan_ints(int np);

@@ -183,22 +183,40 @@ int check_problems(const laph_problem* probs, int n, const laph_solve_opts* opts
 
 }  // namespace
 
+// What pass_layout reads of the problems.
+static std::vector<ProbDesc> pass_descs(const laph_problem* probs, int n, const laph_solve_opts* opts) {
+  std::vector<ProbDesc> d(n);
+  for (int i = 0; i < n; ++i) {
+    d[i].L = probs[i].L;
+    d[i].V3 = d[i].L * d[i].L * d[i].L;
+    d[i].k = round_up(probs[i].nev + opts->guard, kGramTile);
+  }
+  return d;
+}
+
+// The default filter runs a whole pass as one kernel per extent where the batch is small; a column block or a tile
+// other than such a batch's own is a request for the step kernels, the only ones that have them.
+static bool pass_asked(const std::vector<ProbDesc>& d, const laph_solve_opts* opts) {
+  bool variant1 = opts->filter_kernel == 1;
+  if (opts->filter_kernel >= 3)  // what the staged and brick variants cannot take runs as variant 1
+    for (const ProbDesc& p : d) variant1 = variant1 || !cheb_staged_ok(p.L);
+  return variant1 && (opts->block == 0 || opts->block == kSmallBlock) &&
+         (opts->filter_tile == 0 || opts->filter_tile == 128) && pass_small(d);
+}
+
 namespace laph {
 int batch_form(const laph_problem* batch, int n, const laph_solve_opts* opts, int device, BatchForm* f) {
   int sms = 0;
   LAPH_CUDA_TRY(cudaSetDevice(device));
   LAPH_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
   *f = BatchForm{};
-  std::vector<ProbDesc> d(n);  // what pass_layout reads of a problem
+  const std::vector<ProbDesc> d = pass_descs(batch, n, opts);
   long long work = 0, units = 0;
-  for (int i = 0; i < n; ++i) {
-    d[i].L = batch[i].L;
-    d[i].V3 = d[i].L * d[i].L * d[i].L;
-    d[i].k = round_up(batch[i].nev + opts->guard, kGramTile);
-    const int T = d[i].k / kGramTile;
-    work += (long long)d[i].V3 * d[i].k;
-    units += (3LL * d[i].V3 + kGramChunk - 1) / kGramChunk * (T * (T + 1) / 2);
-    f->kmax = std::max(f->kmax, d[i].k);
+  for (const ProbDesc& p : d) {
+    const int T = p.k / kGramTile;
+    work += (long long)p.V3 * p.k;
+    units += (3LL * p.V3 + kGramChunk - 1) / kGramChunk * (T * (T + 1) / 2);
+    f->kmax = std::max(f->kmax, p.k);
   }
   f->gram_split = gram_splits(units);
   // Columns per CTA: 32 unless told otherwise, 16 where 32 would leave too few CTAs per step (below 8e6 site-columns;
@@ -214,12 +232,7 @@ int batch_form(const laph_problem* batch, int n, const laph_solve_opts* opts, in
   };
   f->cols64 = kColsFP64;
   while (f->cols64 > 2 && blocks64(f->cols64) < sms) f->cols64 /= 2;
-  // The default filter runs a whole pass as one kernel per extent where the batch is small; a column block or a tile
-  // other than such a batch's own is a request for the step kernels, the only ones that have them.
-  bool variant1 = opts->filter_kernel == 1;
-  if (opts->filter_kernel >= 3)  // what the staged and brick variants cannot take runs as variant 1
-    for (int i = 0; i < n; ++i) variant1 = variant1 || !cheb_staged_ok(d[i].L);
-  if (variant1 && (opts->block == 0 || opts->block == kSmallBlock) && (opts->filter_tile == 0 || opts->filter_tile == 128)) {
+  if (pass_asked(d, opts)) {
     std::vector<PassClass> pass;
     LAPH_TRY(pass_layout(d, opts->link_prec == LAPH_LINKS_BF16, &pass));
     f->pass = !pass.empty();
@@ -1413,7 +1426,8 @@ int laph_solver_footprint(const laph_problem* probs, int n, const laph_solve_opt
   add(o_tc * 8);
   add(4 * o_kv * 8);                          // dwork
   add(4);                                     // active count
-  add((long long)pass_plan_ints(n) * 4);      // plan of the one-kernel filter pass
+  if (pass_asked(pass_descs(probs, n, opts), opts))
+    add((long long)pass_plan_ints(n) * 4);    // plan of the one-kernel filter pass
   add((long long)(kMlpParams + kMlpNorm) * 4);
   add((long long)n * kMlpIn * 4);
   add((long long)n * (kMlpIn + kMlpOut) * 4);
