@@ -362,8 +362,9 @@ int laph_solver_autotune(const laph_problem* probs, int n, const double* const* 
 
 /* ---- learned Chebyshev window --------------------------------------------
  * A 16 -> 64 -> 64 -> 3 tanh MLP (FP32) maps per-timeslice features -- the
- * smeared plaquette's mean, variance, skewness, excess kurtosis, the 10 Ritz
- * values of a 10-step Lanczos on -Delta (/12), log V3 / log 48^3, k / dim --
+ * smeared plaquette's mean, variance, skewness, excess kurtosis, ten numbers of
+ * the tridiagonal of a 10-step Lanczos on -Delta (/12; the ones the model was
+ * trained on, which are not its eigenvalues), log V3 / log 48^3, k / dim --
  * to (log lambda_cut, lambda_max, degree) of the first filter pass.  No
  * counterpart in the reference, whose window (LAM_L, LAM_C, DEG) is set by
  * hand in parameters.txt.  Parameter layout: W1[64][16] b1[64] W2[64][64]
@@ -378,7 +379,8 @@ int laph_mlp_train(float* params, const float* X, const float* Y, int n, int epo
                    int device);
 /* Model used by window = LAPH_WINDOW_MLP (nfloats = nparams + 38). */
 int laph_solver_set_window_model(laph_solver* s, const float* model, int nfloats);
-/* Features (np x 16) and 10-step Lanczos upper bounds (np) of the last run. */
+/* Features (np x 16; the model's inputs) and 10-step Lanczos upper estimates
+ * theta_max + |beta s| of each spectrum (np) of the last run. */
 int laph_solver_features(laph_solver* s, float* feats, double* bound);
 /* All k Ritz values of problem i after the last run (k returned). */
 int laph_solver_ritz(laph_solver* s, int i, double* theta, int* k);

@@ -142,11 +142,54 @@ __global__ void k_mlp_reduce_adam(float* __restrict__ P, const float* __restrict
 // ---------------------------------------------------------------- features --
 // One CTA (1024 threads) per problem: plaquette power sums of the smeared
 // links and a 10-step FP64 Lanczos on -Delta from a fixed random start
-// (vectors in the scratch block W), then the 10 Ritz values of the Lanczos
-// tridiagonal (Jacobi on thread 0) and the upper bound theta_max + |beta s|.
+// (vectors in the scratch block W), then ten numbers of the Lanczos
+// tridiagonal (thread 0) and the upper estimate theta_max + |beta s| (warp 1).
 // feats[p][16]: 0-3 plaquette mean / variance / skewness / excess kurtosis,
-// 4-13 Ritz values / 12 ascending, 14 log(V3) / log(48^3), 15 k / dim.
-// bound[p]: Lanczos upper bound of the spectrum.
+// 4-13 the ten numbers / 12 ascending, 14 log(V3) / log(48^3), 15 k / dim.
+// bound[p]: Lanczos upper estimate of the spectrum's top.
+//
+// The ten numbers are meant as the tridiagonal's eigenvalues, and the statements
+// below compute these: compiled for the host, without optimisation, or with the
+// loops over k not unrolled, they do.  nvcc 12.9 at -O3 for sm_100a unrolls them
+// into code that does not (its ten numbers do not even add up to the trace).  The
+// learned window's model was trained on what this code returns, so it is kept as
+// it is: other values here need a newly trained model.
+// By one warp: the Lanczos upper estimate of the spectrum's top from the n x n tridiagonal (alpha, beta),
+// theta + |beta_n s|, theta its largest eigenvalue and s the last component of theta's eigenvector.  theta by
+// multisection, a lane per point: x lies above the whole spectrum exactly when every pivot of T - x is negative.  The
+// eigenvector by the rows of (T - theta) v = 0 from the last up, whose pivots are positive for the largest eigenvalue.
+__device__ double lanczos_top(const double* alpha, const double* beta, int n) {
+  const int lane = threadIdx.x & 31;
+  double lo = alpha[0], hi = alpha[0];  // the largest diagonal entry; the largest Gershgorin end
+  for (int i = 0; i < n; ++i) {
+    lo = fmax(lo, alpha[i]);
+    hi = fmax(hi, alpha[i] + (i > 0 ? beta[i - 1] : 0.0) + (i < n - 1 ? beta[i] : 0.0));
+  }
+  for (int round = 0; round < 12; ++round) {  // an interval 33^12 times shorter
+    const double x = lo + (hi - lo) * ((lane + 1) * (1.0 / 33.0));
+    double d = alpha[0] - x;
+    bool above = d < 0.0;
+#pragma unroll 1
+    for (int i = 1; i < n && above; ++i) {
+      d = alpha[i] - x - beta[i - 1] * beta[i - 1] / d;
+      above = d < 0.0;
+    }
+    const int below = __popc(__ballot_sync(0xffffffffu, !above));  // the lower points are not above it
+    const double step = hi - lo, l0 = lo;
+    if (below > 0) lo = l0 + step * (below * (1.0 / 33.0));
+    if (below < 32) hi = l0 + step * ((below + 1) * (1.0 / 33.0));
+  }
+  if (!(beta[n - 1] > 0.0)) return hi;  // an invariant subspace: theta is an eigenvalue
+  double norm2 = 1.0, v = 1.0, e = hi - alpha[n - 1];
+#pragma unroll 1
+  for (int i = n - 1; i > 0; --i) {
+    v *= e / beta[i - 1];
+    norm2 += v * v;
+    e = hi - alpha[i - 1] - beta[i - 1] * beta[i - 1] / e;
+  }
+  return hi + beta[n - 1] / sqrt(norm2);
+}
+
 __global__ void __launch_bounds__(1024) k_features(const ProbDesc* __restrict__ pd, const double2* __restrict__ U64,
                                                    const double* __restrict__ plaq, double2* __restrict__ scratch,
                                                    float* __restrict__ feats, double* __restrict__ bound) {
@@ -235,15 +278,17 @@ __global__ void __launch_bounds__(1024) k_features(const ProbDesc* __restrict__ 
     vp = t;
     beta_prev = bb;
   }
+  if (tid >> 5 == 1) {
+    const double top = lanczos_top(s_alpha, s_beta, kLanczosSteps);
+    if (tid == 32) bound[p] = top;
+  }
   if (tid == 0) {
     // Jacobi on the 10 x 10 tridiagonal
     constexpr int n = kLanczosSteps;
-    double A[n][n], Q[n][n];
+    double A[n][n];
     for (int a = 0; a < n; ++a)
-      for (int b = 0; b < n; ++b) {
+      for (int b = 0; b < n; ++b)
         A[a][b] = (a == b) ? s_alpha[a] : ((b == a + 1) ? s_beta[a] : ((a == b + 1) ? s_beta[b] : 0.0));
-        Q[a][b] = (a == b) ? 1.0 : 0.0;
-      }
     for (int sweep = 0; sweep < 30; ++sweep) {
       double off = 0.0;
       for (int a = 0; a < n; ++a)
@@ -264,11 +309,6 @@ __global__ void __launch_bounds__(1024) k_features(const ProbDesc* __restrict__ 
             const double ak = A[a][k], bk = A[b][k];
             A[a][k] = c * ak - s * bk;
             A[b][k] = s * ak + c * bk;
-          }
-          for (int k = 0; k < n; ++k) {
-            const double qa = Q[k][a], qb = Q[k][b];
-            Q[k][a] = c * qa - s * qb;
-            Q[k][b] = s * qa + c * qb;
           }
         }
     }
@@ -300,8 +340,6 @@ __global__ void __launch_bounds__(1024) k_features(const ProbDesc* __restrict__ 
     for (int a = 0; a < n; ++a) f[4 + a] = (float)(th[idx[a]] / 12.0);
     f[14] = (float)(log((double)d.V3) / log(48.0 * 48.0 * 48.0));
     f[15] = (float)((double)d.k / d.dim);
-    const int top = idx[n - 1];
-    bound[p] = th[top] + fabs(s_beta[n - 1] * Q[n - 1][top]);
   }
 }
 
@@ -312,12 +350,11 @@ __global__ void __launch_bounds__(1024) k_features(const ProbDesc* __restrict__ 
 //             because its block is still a random one (margin calibrated on
 //             training lattices, laph_solve_opts.window_margin);
 //   lam_max stays the exact bound 12 of the spectrum of -Delta (or the fixed
-//             one): prediction 1 learns the 10-step Lanczos estimate of the
-//             top, which lies well below the true top (9.3-10.6 against
-//             11.5+ on 16^3-32^3 smeared fields), and a window whose top is
-//             below the spectrum's lets T_m amplify the highest eigenvectors
-//             past the wanted ones -- solves with it did not converge in 300
-//             passes -- so it is not used;
+//             one): a window whose top is below the spectrum's lets T_m
+//             amplify the highest eigenvectors past the wanted ones (solves
+//             with such a top did not converge in 300 passes), and neither a
+//             prediction nor the Lanczos estimate of the top is a guaranteed
+//             bound, so prediction 1 is not used;
 //   degree  = prediction 2, clamped to [8, 64], written to out_deg.
 __global__ void k_window_apply(const ProbDesc* __restrict__ pd, ProbState* __restrict__ ps, int np,
                                const float* __restrict__ O, const float* __restrict__ norm,

@@ -3,13 +3,15 @@
 The block solver's first filter pass needs a damped interval [lambda_cut,
 lambda_max] and a degree before any Ritz value exists.  A 16 -> 64 -> 64 -> 3
 MLP (FP32, trained and evaluated by this library's own CUDA kernels) maps
-per-timeslice features -- smeared-plaquette moments and the Ritz values of a
+per-timeslice features -- smeared-plaquette moments and ten numbers of a
 10-step Lanczos, computed on the device by the solver -- to
 
     target 0: log of the window cut the non-learned (Lanczos/adaptive) solver
               converges to, i.e. its final largest Ritz value theta_{k-1};
-    target 1: lambda_max (the 10-step Lanczos upper bound; reported only: the
-              solver keeps the exact bound 12 of the spectrum of -Delta);
+    target 1: lambda_max (the 10-step Lanczos upper estimate; not used: the
+              solver keeps the exact bound 12 of the spectrum of -Delta.  The
+              model in data/ was trained when the estimate came out too low,
+              so its prediction 1 means nothing);
     target 2: a filter degree: the smallest m that damps the slowest wanted
               pair theta_{nev-1} relative to theta_{k-1} by FIRST_PASS_GAIN.
 
