@@ -201,7 +201,7 @@ def autotune_cfg(cfg, batch, device, nsample, cache):
                             opts=make_opts(cfg), model=model, device=device, cache=cache)
     res["seconds"] = time.perf_counter() - t0
     res["sample_timeslices"] = min(nsample, len(batch))
-    res["before"] = {"deg": cfg["deg"], "block": cfg.get("block", 0) or 32, "guard": cfg["guard"],
+    res["before"] = {"deg": cfg["deg"], "block": cfg.get("block", 0), "guard": cfg["guard"],
                      "tile": cfg.get("tile", 0) or 128}
     cfg["deg"], cfg["block"], cfg["guard"], cfg["tile"] = opts.deg, opts.block, opts.guard, opts.filter_tile
     return res
@@ -214,6 +214,21 @@ def make_solver(cfg, device, batch):
     for i, (a1, a2) in enumerate(cfg.get("scan") or []):
         s.set_smear(i, a1, a2)  # the batched tune_hyp scan: one copy of the timeslice per grid point
     return s
+
+
+def solver_form(solver):
+    """(columns per CTA of the filter, whether its passes run as one kernel each) of a solver."""
+    import ctypes
+    import laph_eigsys_b200 as lb
+    block, one = ctypes.c_int(), ctypes.c_int()
+    lb.check(lb.lib.laph_solver_form(solver._h, ctypes.byref(block), ctypes.byref(one)), "laph_solver_form")
+    return block.value, bool(one.value)
+
+
+def link_model(cfg, block, one):
+    """The links' share of the filter's byte model."""
+    per = 112 if cfg["link_prec"] == "bf16" else 216
+    return f"links ({per} B per site) once per pass" if one else f"{per}/{block} B"
 
 
 def cpu_reference_step(cfg, links_ts, lam_c, deg_ref, threads, L=None, nev=None, keep=False):
@@ -394,7 +409,6 @@ def solve_config(cfg, device, reps=1, window=None, link_prec=None, wave=None, pa
     torch.cuda.synchronize()
     ms = e0.elapsed_time(e1) / reps
     hbm, src = peaks()
-    kb = cfg.get("block") or 32
     out = {"workload": workload_config(cfg)["workload"], "timeslices": len(batch), "status": st,
            "value": len(batch) / (ms / 1e3), "unit": "timeslices/s", "ms_per_solve": ms,
            "outer_iterations": max(r["iters"] for r in res), "max_resid": max(r["max_resid"] for r in res),
@@ -403,7 +417,7 @@ def solve_config(cfg, device, reps=1, window=None, link_prec=None, wave=None, pa
            "filter": {"ms_per_solve": filt_ms / reps, "achieved_gbs": fb[0] / (filt_ms / 1e3) / 1e9,
                       "frac": fb[0] / (filt_ms / 1e3) / 1e9 / hbm,
                       "frac_s8d": fb[1] / (filt_ms / 1e3) / 1e9 / hbm, "peak_gbs": hbm, "peak_source": src,
-                      "bytes_model_s8d": f"72 + {112 if cfg['link_prec'] == 'bf16' else 216}/{kb} B"}}
+                      "bytes_model_s8d": f"72 B + {link_model(cfg, *solver_form(solver))}"}}
     if parity and not no_cpu:
         import oracle as orc
         orc.set_threads(os.cpu_count() or 1)
@@ -461,7 +475,7 @@ def workload_config(cfg):
     return {"workload": f"{shape}, eps {cfg['eps']} {cfg['smear']} {cfg['iters']}x{cfg['p1']}, "
                         f"+{cfg['guard']} guard, resid<=1e-9",
             "L": cfg["L"], "timeslices": cfg["T"], "nev": cfg["nev"], "guard": cfg["guard"], "deg": cfg["deg"],
-            "block": cfg.get("block") or 32, "tile": cfg.get("tile") or 128,
+            "block": cfg.get("block_used") or cfg.get("block") or 32, "tile": cfg.get("tile") or 128,
             "window": cfg.get("window", "mlp"),
             "links": cfg["link_prec"], "filter": "fp32", "rayleigh_ritz": "fp64",
             "l2": "inputs larger than L2 (each 64-timeslice block of vectors is 8 GB)"}
@@ -763,14 +777,14 @@ def main():
     # algorithmic bytes of the timed filter passes, counted by the solver pass by pass (each pass's own degree,
     # its unlocked columns and column blocks): what the correction-form recurrence moves, and the unit
     # of one step Y = 2BX - Z (72 B per site-vector-step + links once per column block)
-    kb = cfg["block"] or 32
-    link_b = 112 if cfg["link_prec"] == "bf16" else 216
+    kb, one_kernel = solver_form(solver)
+    cfg["block_used"] = kb
     alg_bytes, alg_s8d = fbytes_tot
     hbm, src = peaks()
     achieved = alg_bytes / (filt_ms / 1000.0) / 1e9 if filt_ms > 0 else None
     achieved_s8d = alg_s8d / (filt_ms / 1000.0) / 1e9 if filt_ms > 0 else None
     fk = cfg.get("filter_kernel", 1)
-    kname = ({2: "k_cheb_mrhs3", 3: "k_cheb_mrhs4", 4: "k_cheb_mrhs5", 5: "k_cheb_mrhs6"}.get(fk, "k_cheb_mrhs2")) if fk >= 1 and kb <= 64 else "k_cheb_mrhs"
+    kname = "k_cheb_pass" if one_kernel else ({2: "k_cheb_mrhs3", 3: "k_cheb_mrhs4", 4: "k_cheb_mrhs5", 5: "k_cheb_mrhs6"}.get(fk, "k_cheb_mrhs2")) if fk >= 1 and kb <= 64 else "k_cheb_mrhs"
     roofline = {"kernel": f"{kname} (lap_cheb_mrhs)", "bound": "hbm", "achieved": achieved, "peak": hbm,
                 "unit": "GB/s", "frac": achieved / hbm if achieved else None, "peak_source": src,
                 "traffic": NCU_TRAFFIC_RATIO * alg_bytes / max(flaunch, 1) if kname == "k_cheb_mrhs2" else None,
@@ -779,7 +793,7 @@ def main():
                 "bytes_per_launch": alg_bytes / max(flaunch, 1),
                 "filter_share_of_step": filt_ms / ms if ms > 0 else None,
                 "achieved_s8d": achieved_s8d, "frac_s8d": achieved_s8d / hbm if achieved_s8d else None,
-                "bytes_model_s8d": f"72 + {link_b}/{kb} B per site-vector-step"}
+                "bytes_model_s8d": f"72 B + {link_model(cfg, kb, one_kernel)} per site-vector-step"}
 
     # ---- e2e through the public API with host buffers ----------------------
     e2e = None

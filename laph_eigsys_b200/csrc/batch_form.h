@@ -22,6 +22,8 @@ extern "C" {
 // laph_solver_create for probs[0..n), with the kernels of batch[0..nbatch), of which they are a sample.
 int laph_solver_create_for(laph_solver** out, const laph_problem* probs, int n, const laph_solve_opts* opts, int device,
                            const laph_problem* batch, int nbatch);
+// Columns per CTA of the solver's filter, and whether its passes run as one kernel each.
+int laph_solver_form(laph_solver* s, int* block, int* pass);
 // Blocks wider than `width` run their Jacobi in global memory, as they do on a device without room for their clusters
 // (for the tests; before the solver's first run).
 int laph_solver_limit_jacobi(laph_solver* s, int width);

@@ -1285,6 +1285,16 @@ int laph_solver_timings(laph_solver* s, double* ms4) {
   return LAPH_OK;
 }
 
+int laph_solver_form(laph_solver* s, int* block, int* pass) {
+  if (!s || !block || !pass) {
+    set_error("laph_solver_form: bad argument");
+    return LAPH_EINVAL;
+  }
+  *block = s->kb;
+  *pass = !s->pass.empty();
+  return LAPH_OK;
+}
+
 int laph_solver_limit_jacobi(laph_solver* s, int width) {
   if (!s || s->ran || width < 0) {
     set_error("laph_solver_limit_jacobi: bad argument or solver has run");

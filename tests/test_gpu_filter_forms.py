@@ -2,6 +2,7 @@
 a tile other than such a batch's own (16 columns, 128 sites) takes the kernels that run step by step, which alone have
 them.  The step kernels then stay covered on small lattices: every tile with both link types, the staged and the brick
 variant, and the bounds-checked build, all bit for bit."""
+import ctypes
 import json
 import os
 import subprocess
@@ -34,6 +35,24 @@ def _same(a, b):
 
 
 PROBS = [(10, 24), (12, 30)]
+
+
+def _form(gpu, probs, **kw):
+    s = gpu.Solver(probs, **kw)
+    block, one = ctypes.c_int(), ctypes.c_int()
+    gpu.check(gpu.lib.laph_solver_form(s._h, ctypes.byref(block), ctypes.byref(one)), "laph_solver_form")
+    s.close()
+    return block.value, one.value
+
+
+def test_a_solver_says_which_form_it_runs(gpu):
+    assert _form(gpu, PROBS) == (16, 1)
+    assert _form(gpu, PROBS, block=16, filter_tile=128) == (16, 1)
+    assert _form(gpu, PROBS, filter_tile=64) == (16, 0)
+    assert _form(gpu, PROBS, block=8) == (8, 0)
+    assert _form(gpu, PROBS, filter_kernel=2) == (16, 0)
+    assert _form(gpu, [(32, 120)]) == (16, 0)  # 4.5e6 site-columns
+    assert _form(gpu, [(32, 120)] * 2) == (32, 0)
 
 
 def test_own_block_and_tile_keep_the_one_kernel_pass(gpu):
