@@ -343,7 +343,8 @@ int laph_autotune_search(const int* deg_c, int nd, const int* block_c, int nb, c
  * FP64 host links in `layout`; each setting is timed as the faster of two runs
  * of a solver over the sample (the first also captures its CUDA graphs), a
  * setting that does not converge within opts->max_it is dropped.  The sample's
- * solves run the kernels that the whole batch takes.  model /
+ * solves run the kernels that the whole batch takes, and repeat the sample up to
+ * 4e7 site-columns or n problems.  model /
  * nmodel: the window model (as laph_solver_set_window_model) when
  * opts->window is LAPH_WINDOW_MLP, else ignored (may be NULL).  Candidates:
  * deg 40, 48, 56, 60, 64, 72, 80, 96 (start: opts->deg, or 60 if <= 1), block 8, 16, 32, 64

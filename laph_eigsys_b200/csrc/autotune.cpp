@@ -16,7 +16,8 @@
 // at most once.  laph_solver_autotune times each setting as a real solve of a
 // sample of the batch (the faster of two runs of one solver: the first also
 // captures the CUDA graphs), run by the kernels the whole batch takes
-// (batch_form.h), and keeps the result in an optional cache file, one line per
+// (batch_form.h) and repeated until it is large enough that the serial parts of a
+// solve weigh little, as they do in the batch, and keeps the result in an optional cache file, one line per
 // device and batch shape, so a production run tunes once.  A batch whose filter
 // runs whole passes as one kernel has no block and no tile to tune.
 #include <cuda_runtime.h>
@@ -41,10 +42,16 @@ using laph::set_error;
 namespace {
 
 constexpr double kTuneMargin = 0.01;  // a candidate must be this much faster to replace the best
+// A trial solves the sample, repeated up to this many site-columns (of nev + guard rounded up to 32) or the batch's size:
+// the features, the Cholesky and the Jacobi take about the same time for 4 problems as for 64, so a small sample favours
+// few passes on wide blocks.  32^3, nev 120, ms per timeslice with guard 8 and 16: 4 timeslices 38.9 and 39.0, 8 (4e7)
+// 35.8 and 37.0, 16 35.5 and 37.2, the batch of 64 34.8 and 37.0.  A run of that size takes about 0.3 s.
+constexpr long long kTuneWork = 40000000;
 
 struct SampleCtx {
   const laph_problem* probs;
   int n, ns;  // the batch, and how many of it are the sample
+  int m;      // problems of a trial: the sample, repeated
   const double* const* links;
   int layout;
   laph_solve_opts base;
@@ -64,17 +71,23 @@ double sample_trial(void* user, int deg, int block, int guard) {
   o.guard = guard;
   o.filter_tile = c->tile;
   laph_solver* s = nullptr;
-  int st = laph_solver_create_for(&s, c->probs, c->ns, &o, c->device, c->probs, c->n);
+  std::vector<laph_problem> trial(c->m);
+  for (int i = 0; i < c->m; ++i) trial[i] = c->probs[i % c->ns];
+  int st = laph_solver_create_for(&s, trial.data(), c->m, &o, c->device, c->probs, c->n);
+  if (st == LAPH_ENOMEM && c->m > c->ns) {  // no room for more than the sample itself
+    c->m = c->ns;
+    st = laph_solver_create_for(&s, trial.data(), c->m, &o, c->device, c->probs, c->n);
+  }
   c->last_status = st;
   if (st != LAPH_OK) return -1.0;
   double best = -1.0;
   if (o.window == LAPH_WINDOW_MLP) st = laph_solver_set_window_model(s, c->model, c->nmodel);
-  for (int i = 0; i < c->ns && st == LAPH_OK; ++i) st = laph_solver_set_links(s, i, c->links[i], c->layout, 0);
+  for (int i = 0; i < c->m && st == LAPH_OK; ++i) st = laph_solver_set_links(s, i, c->links[i % c->ns], c->layout, 0);
   for (int rep = 0; rep < 2 && st == LAPH_OK; ++rep) {
     st = laph_solver_run(s, nullptr);
     double ms[4] = {0, 0, 0, 0};
     if (st == LAPH_OK && laph_solver_timings(s, ms) == LAPH_OK && ms[3] > 0.0) {
-      const double per = ms[3] / c->ns;
+      const double per = ms[3] / c->m;
       best = best < 0.0 ? per : std::min(best, per);
     }
   }
@@ -245,7 +258,17 @@ int laph_solver_autotune(const laph_problem* probs, int n, const double* const* 
   if (gmin != guard0 && gmin != guard0 + 32 && ((probs[0].nev + gmin + 31) / 32 != (probs[0].nev + guard0 + 31) / 32))
     guards.push_back(gmin);
   const int tile0 = opts->filter_tile > 0 ? opts->filter_tile : 128;
-  SampleCtx ctx{probs, n, ns, links, layout, *opts, model, nmodel, device, LAPH_OK, tile0};
+  int m = ns;
+  if (solvable && opts->guard >= 0) {
+    long long work = 0;
+    auto add = [&](int i) {
+      const long long L = probs[i % ns].L;
+      work += L * L * L * ((probs[i % ns].nev + opts->guard + 31) / 32 * 32);
+    };
+    for (int i = 0; i < ns; ++i) add(i);
+    for (; m < n && work < kTuneWork; ++m) add(m);
+  }
+  SampleCtx ctx{probs, n, ns, m, links, layout, *opts, model, nmodel, device, LAPH_OK, tile0};
   int st = laph_autotune_search(degs, 8, blocks, form.pass ? 0 : 4, guards.data(), (int)guards.size(), deg0, block0, guard0,
                                 sample_trial, &ctx, out);
   if (st != LAPH_OK) {
