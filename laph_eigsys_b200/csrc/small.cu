@@ -31,6 +31,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <mutex>
 
 #include "dense.cuh"
 
@@ -906,8 +907,19 @@ int small_init() {
 }
 
 // A cluster of 16 CTAs of up to 215 KB, or of 8 of up to 210 KB, may have no room on the device (fewer SMs in every GPC,
-// as in a partitioned one); its blocks then take the global-memory form.
+// as in a partitioned one); its blocks then take the global-memory form.  Asked once per device: the two questions take
+// 0.4 ms, a tenth of creating a small solver.
 int small_jacobi_width(int* n) {
+  static std::mutex mu;
+  static int width[64];
+  static bool known[64];
+  int dev = 0;
+  LAPH_CUDA_TRY(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lk(mu);
+  if (dev < 64 && known[dev]) {
+    *n = width[dev];
+    return LAPH_OK;
+  }
   auto fits = [](const void* fn, int c, int smem) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(c);
@@ -929,6 +941,10 @@ int small_jacobi_width(int* n) {
   *n = !fits((const void*)k_jacobi<8, true, false>, 8, 4 * kJacSmemN8 * kJacSmemN8)       ? 0
        : !fits((const void*)k_jacobi<16, true, false>, 16, 2 * kJacSmemN16 * kJacSmemN16) ? kJacSmemN8
                                                                                           : kJacSmemN16;
+  if (dev < 64) {
+    width[dev] = *n;
+    known[dev] = true;
+  }
   return LAPH_OK;
 }
 
