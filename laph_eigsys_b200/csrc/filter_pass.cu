@@ -331,21 +331,21 @@ __global__ void __launch_bounds__(kPassThreads, 2)
 
 size_t pass_plan_ints(int np) { return plan_ctr(np) + (size_t)kPassClasses * kMaxTeams * kPassLine; }
 
-bool pass_small(const std::vector<ProbDesc>& probs) {
-  long long work = 0;
-  int extents = 0, seen[kPassClasses] = {};
-  for (const ProbDesc& d : probs) {
-    work += (long long)d.V3 * d.k;
-    if (std::find(seen, seen + extents, d.L) != seen + extents) continue;
-    if (extents == kPassClasses) return false;
-    seen[extents++] = d.L;
-  }
-  return work <= kPassMaxWork;
+void PassSize::add(int L, int k) {
+  work += (long long)L * L * L * k;
+  int c = 0;
+  while (c < extents && c < kPassClasses && seen[c] != L) ++c;
+  if (c < extents && c < kPassClasses) return;
+  if (c < kPassClasses) seen[c] = L;
+  extents = c + 1;  // kPassClasses + 1: one too many, and stays so
 }
+bool PassSize::small() const { return work <= kPassMaxWork && extents <= kPassClasses; }
 
 int pass_layout(const std::vector<ProbDesc>& probs, int bf16, std::vector<PassClass>* out) {
   out->clear();
-  if (!pass_small(probs)) return LAPH_OK;
+  PassSize size;
+  for (const ProbDesc& d : probs) size.add(d.L, d.k);
+  if (!size.small()) return LAPH_OK;
   int dev = 0, sms = 0, occ = 0;
   const void* fn = bf16 ? (const void*)k_cheb_pass<__nv_bfloat162> : (const void*)k_cheb_pass<float2>;
   LAPH_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kPassSmem));

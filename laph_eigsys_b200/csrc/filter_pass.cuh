@@ -19,7 +19,13 @@ struct PassClass {
 // ones (an extent whose sites outnumber the co-resident threads, or more than
 // kPassClasses extents).
 constexpr int kPassClasses = 4;
-bool pass_small(const std::vector<ProbDesc>& probs);  // few enough site-columns and extents for it (reads L, V3 and k)
+// Have the problems few enough site-columns and extents for it?  Fed one by one.
+struct PassSize {
+  long long work = 0;
+  int extents = 0, seen[kPassClasses] = {};
+  void add(int L, int k);
+  bool small() const;
+};
 int pass_layout(const std::vector<ProbDesc>& probs, int bf16, std::vector<PassClass>* out);
 // ints of plan scratch for np problems
 size_t pass_plan_ints(int np);

@@ -183,25 +183,18 @@ int check_problems(const laph_problem* probs, int n, const laph_solve_opts* opts
 
 }  // namespace
 
-// What pass_layout reads of the problems.
-static std::vector<ProbDesc> pass_descs(const laph_problem* probs, int n, const laph_solve_opts* opts) {
-  std::vector<ProbDesc> d(n);
-  for (int i = 0; i < n; ++i) {
-    d[i].L = probs[i].L;
-    d[i].V3 = d[i].L * d[i].L * d[i].L;
-    d[i].k = round_up(probs[i].nev + opts->guard, kGramTile);
-  }
-  return d;
-}
-
 // The default filter runs a whole pass as one kernel per extent where the batch is small; a column block or a tile
 // other than such a batch's own is a request for the step kernels, the only ones that have them.
-static bool pass_asked(const std::vector<ProbDesc>& d, const laph_solve_opts* opts) {
+static bool pass_asked(const laph_problem* probs, int n, const laph_solve_opts* opts) {
   bool variant1 = opts->filter_kernel == 1;
-  if (opts->filter_kernel >= 3)  // what the staged and brick variants cannot take runs as variant 1
-    for (const ProbDesc& p : d) variant1 = variant1 || !cheb_staged_ok(p.L);
+  PassSize size;
+  for (int i = 0; i < n; ++i) {
+    size.add(probs[i].L, round_up(probs[i].nev + opts->guard, kGramTile));
+    // what the staged and brick variants cannot take runs as variant 1
+    if (opts->filter_kernel >= 3 && !cheb_staged_ok(probs[i].L)) variant1 = true;
+  }
   return variant1 && (opts->block == 0 || opts->block == kSmallBlock) &&
-         (opts->filter_tile == 0 || opts->filter_tile == 128) && pass_small(d);
+         (opts->filter_tile == 0 || opts->filter_tile == 128) && size.small();
 }
 
 namespace laph {
@@ -210,7 +203,12 @@ int batch_form(const laph_problem* batch, int n, const laph_solve_opts* opts, in
   LAPH_CUDA_TRY(cudaSetDevice(device));
   LAPH_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
   *f = BatchForm{};
-  const std::vector<ProbDesc> d = pass_descs(batch, n, opts);
+  std::vector<ProbDesc> d(n);  // what pass_layout reads of a problem
+  for (int i = 0; i < n; ++i) {
+    d[i].L = batch[i].L;
+    d[i].V3 = d[i].L * d[i].L * d[i].L;
+    d[i].k = round_up(batch[i].nev + opts->guard, kGramTile);
+  }
   long long work = 0, units = 0;
   for (const ProbDesc& p : d) {
     const int T = p.k / kGramTile;
@@ -232,7 +230,7 @@ int batch_form(const laph_problem* batch, int n, const laph_solve_opts* opts, in
   };
   f->cols64 = kColsFP64;
   while (f->cols64 > 2 && blocks64(f->cols64) < sms) f->cols64 /= 2;
-  if (pass_asked(d, opts)) {
+  if (pass_asked(batch, n, opts)) {
     std::vector<PassClass> pass;
     LAPH_TRY(pass_layout(d, opts->link_prec == LAPH_LINKS_BF16, &pass));
     f->pass = !pass.empty();
@@ -1436,7 +1434,7 @@ int laph_solver_footprint(const laph_problem* probs, int n, const laph_solve_opt
   add(o_tc * 8);
   add(4 * o_kv * 8);                          // dwork
   add(4);                                     // active count
-  if (pass_asked(pass_descs(probs, n, opts), opts))
+  if (pass_asked(probs, n, opts))
     add((long long)pass_plan_ints(n) * 4);    // plan of the one-kernel filter pass
   add((long long)(kMlpParams + kMlpNorm) * 4);
   add((long long)n * kMlpIn * 4);

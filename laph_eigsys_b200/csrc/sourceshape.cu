@@ -29,7 +29,8 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
-#include <vector>
+#include <memory>
+#include <new>
 
 #include "batch.cuh"
 #include "bulk.cuh"
@@ -411,12 +412,16 @@ int sourceshape_device(const double2* V, int L, int nev, const double* evals, do
 // The bins of sourceshape_device to the host, once its work on st is done.
 int sourceshape_copy(const double* dpsi, int L, double* psi, cudaStream_t st) {
   const int H = L / 2, Nc = H * H * H;
-  std::vector<double> h(Nc + 1);  // bins and flag in one copy
-  LAPH_CUDA_TRY(cudaMemcpyAsync(h.data(), dpsi, sizeof(double) * (Nc + 1), cudaMemcpyDeviceToHost, st));
+  std::unique_ptr<double[]> h(new (std::nothrow) double[Nc + 1]);  // bins and flag in one copy
+  if (!h) {
+    set_error("laph_sourceshape: host allocation failed");
+    return LAPH_ENOMEM;
+  }
+  LAPH_CUDA_TRY(cudaMemcpyAsync(h.get(), dpsi, sizeof(double) * (Nc + 1), cudaMemcpyDeviceToHost, st));
   LAPH_CUDA_TRY(cudaStreamSynchronize(st));
   int gave_up;
   std::memcpy(&gave_up, &h[Nc], sizeof gave_up);
-  std::memcpy(psi, h.data(), sizeof(double) * Nc);
+  std::memcpy(psi, h.get(), sizeof(double) * Nc);
   return laph_sourceshape_status(gave_up);
 }
 
