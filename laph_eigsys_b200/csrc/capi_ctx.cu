@@ -177,8 +177,8 @@ int laph_set_links(laph_ctx* c, const double* links, int layout) {
   }
   // The spatial links go through the two halves of the pinned staging buffer: while one half's copy is in flight the
   // host threads check and pack the next sites into the other (against single-threaded reorders and pageable copies here
-  // and in laph_get_links, a 24^3 timeslice's set-up with HYP smearing and plaquette takes 0.54 instead of 5.4 ms).  The reorder on the device runs last, so links with a
-  // non-finite entry leave the context's as they were.
+  // and in laph_get_links, a 24^3 timeslice's set-up with HYP smearing and plaquette takes 0.52 instead of 5.0 ms).  The
+  // reorder on the device runs last, so links with a non-finite entry leave the context's as they were.
   const int V3 = c->g.V3;
   const long long chunk = (long long)(c->half / 27);
   double2* raw = c->dec;  // [site][27]; the decorated links' storage is free outside laph_smear

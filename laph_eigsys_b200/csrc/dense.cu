@@ -4,8 +4,9 @@
 //   (small.cu: from G and H to the Ritz values, the rotation's coefficients C
 //   and the next Chebyshev window)
 //   k_rotate      V = W C
-//   k_residual64  R = (-Delta) V - V diag(theta) (FP64 stencil), S = -2 c_hop R
-//                 (FP32), residual partial sums
+//   k_residual64_cols  R = (-Delta) V - V diag(theta) (FP64 stencil), S = -2 c_hop R
+//                 (FP32), residual partial sums (k_residual64, one thread per site
+//                 and column, with LAPH_RESID_KERNEL=0)
 //   k_resid       residual norms, convergence mask
 // Columns [0, c0) of a problem (whole tiles of locked Ritz vectors) are frozen:
 // the Gram skips frozen x frozen tiles, the small problem projects the active

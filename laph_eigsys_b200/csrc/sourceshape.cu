@@ -115,7 +115,7 @@ __device__ __forceinline__ void ss_bin(double* bins, double f, int ys, int xs, i
 // bins are zeroed and flushed once per CTA instead of once per tile.  The rows come
 // by the bulk copy engine, a row of a tile (1536 B) per copy, as the per-thread copies
 // they replace took issue slots from the MMAs.  Measured through laph_sourceshape,
-// allocations included, 120 vectors: 32^3 27.7 -> 21.5 ms, 24^3 6.1 -> 5.1 ms; without
+// allocations included, 120 vectors, medians: 32^3 27.9 -> 21.5 ms, 24^3 6.2 -> 5.0 ms; without
 // the bulk copies 22.5 and 5.2 ms.  A third ring stage and steps of 8 are
 // as good as 2 stages of 16 (21.8 ms) and better than 5 of 4 (23.6 ms).
 constexpr int kSsPitch = kSsRows + 2;                // double2 per ring row: fragment reads hit every bank once

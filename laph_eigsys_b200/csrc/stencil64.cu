@@ -111,9 +111,9 @@ int cheb64(const double2* U, int L, double lam_l, double lam_c, int deg, const d
 //  - a lattice of at most 2048 sites is one cluster of 16 CTAs, whose barrier is
 //    the hardware's (about 0.5 us against 1.3 us through a counter in L2); at 16^3
 //    it would be 256 sites per SM, 44.5 us against 39.4 us for 128 CTAs.
-// us per product (deg 8 at 8^3, else 12), before -> now: 8^3 43.4 -> 22.3, 12^3
-// 62.5 -> 35.2, 16^3 62.5 -> 39.4, 24^3 63.9 -> 42.0, 32^3 70.4 -> 49.9, 36^3
-// 118.8 -> 98, 48^3 165.7 -> 133.
+// us per product (deg 8 at 8^3, else 12; the call from Python included), before -> now:
+// 8^3 43.6 -> 22.0, 12^3 61.5 -> 34.7, 16^3 61.6 -> 39.3, 24^3 63.4 -> 42.2, 32^3
+// 69.8 -> 49.7, 36^3 115 -> 101, 48^3 168 -> 135.
 
 // Grid barrier with a bounded wait, one atomic per CTA and arrival: every CTA
 // adds 1 to the counter except CTA 0, which adds 2^31 - (nblk - 1), so the
